@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(128) lu_kernel(long long n_sys, const R* __res
   const int l = lane % W;
   const int g = threadIdx.x / W;
   const int subs = blockDim.x / W;
-  // per sub-warp: the solve scratch [lu_scratch_len(N)] (pivot rows, or the whole system), solution [N]
+  // per sub-warp: the solve scratch [lu_scratch_len(N)] (pivot rows, or the whole system), pivot reciprocals [N]
   cx<R>* sx = dev::view<R>(smem) + (size_t)g * (dev::lu_scratch_len(N) + N);
   cx<R>* sol = sx + dev::lu_scratch_len(N);
   for (long long s0 = (long long)blockIdx.x * subs; s0 < n_sys; s0 += (long long)gridDim.x * subs) {
@@ -40,10 +40,10 @@ __global__ void __launch_bounds__(128) lu_kernel(long long n_sys, const R* __res
       row[j] = mine ? dev::mk(A[2 * ((s * N + l) * N + j)], A[2 * ((s * N + l) * N + j) + 1]) : dev::mk(R(0), R(0));
     });
     const cx<R> rhs = mine ? dev::mk(b[2 * (s * N + l)], b[2 * (s * N + l) + 1]) : dev::mk(R(0), R(0));
-    dev::lu_solve<R, N, W>(row, rhs, l, sx, sol);
+    const cx<R> v = dev::lu_solve<R, N, W>(row, rhs, l, sx, sol);
     if (mine) {
-      z[2 * (s * N + l)] = sol[l].re;
-      z[2 * (s * N + l) + 1] = sol[l].im;
+      z[2 * (s * N + l)] = v.re;
+      z[2 * (s * N + l) + 1] = v.im;
     }
     __syncwarp(dev::kFull);
   }

@@ -313,38 +313,53 @@ __device__ __forceinline__ void static_for(F&& f) {
   }
 }
 
-// Partial-pivot LU + back substitution, one row per lane, rows in registers.
-// The pivot is found by an integer max butterfly over the sub-warp.  A
-// zero pivot skips that column's elimination and leaves a non-finite
-// solution, as in the reference.  Solution lands in sol[0..N); sx holds two
-// pivot-row buffers of N+1 entries (row + right-hand side), used by
-// alternate columns so that one __syncwarp per column suffices.
-//
-// Two code shapes with the same operations in the same order:
-//   LU_UNROLLED  every column unrolled at compile time (template recursion, so
-//                the row stays in registers at any N; code grows as N^2),
-//   LU_ROLLED    a rolled column loop whose row update runs over all N entries
-//                predicated on j > i (N^2 instead of N^2/2 issue slots, code
-//                linear in N).
-// pragma unroll alone gives up above N = 16 and moves the row to local memory.
-//   LU_SERIAL    (N <= 3) every lane of the sub-warp gathers the whole system
-//                through shared memory and eliminates it in its registers, rows
-//                swapped by selects: no pivot search across lanes and no
-//                broadcast per column, so a lone small system's solve is a short
-//                chain (the single-instance P3P case is latency bound).
-constexpr int LU_UNROLLED = 0, LU_ROLLED = 1, LU_SERIAL = 2;
-#ifndef GHC_LU_LARGE
-#define GHC_LU_LARGE LU_UNROLLED
-#endif
+// Partial-pivot LU + back substitution, one row per lane, rows in registers.  A zero pivot skips
+// that column's elimination and leaves a non-finite solution, as in the reference.  Two forms, the
+// operations of every entry in the oracle's order:
+//   LU_GROUPED  columns in groups of lu_group(N), each group one rolled loop whose body eliminates
+//               the row's first entry and shifts the row down by one, so that a column needs no
+//               compile-time index: the code is one body per group instead of one per column
+//               (N = 12: 0.5 K instead of 1.9 K instructions).  The pivot rows stay in shared
+//               memory, where the back substitution finds them; pivoted lanes go on computing
+//               values that nothing reads, so the update has no branch.  What bounded the LU with
+//               every column unrolled was fetching its code (gen-3v-4pt: 2.0 of 8.9 cycles per
+//               issue); grouped, the same tracker issues in 62 instead of 51 % of the cycles.
+//               Measured against it (B200, default launch choice): gen-3v-4pt FP64 101.9 -> 92.8 ms
+//               (512 hypotheses), mixed 46.6 -> 39.0 (251), CY 103.2 -> 96.8 (128), 30x30 FP64
+//               126.8 -> 117.0 (48), mixed 86.8 -> 75.8 (37); 5-point equal (-0.4 %).
+//   LU_SERIAL   (N <= 3) every lane of the sub-warp gathers the whole system through shared memory
+//               and eliminates it in its registers, rows swapped by selects: no pivot search across
+//               lanes and no broadcast per column, so a lone small system's solve is a short chain
+//               (the single-instance P3P case is latency bound).
+constexpr int LU_GROUPED = 0, LU_SERIAL = 2;
 #ifndef GHC_LU_SERIAL_MAX_N
 #define GHC_LU_SERIAL_MAX_N 3
 #endif
 template <int N>
-constexpr int kLuForm = N <= GHC_LU_SERIAL_MAX_N ? LU_SERIAL : N <= 16 ? LU_UNROLLED : GHC_LU_LARGE;
-// complex values of the per-sub-warp solve scratch sx: two pivot rows with their right-hand sides,
+constexpr int kLuForm = N <= GHC_LU_SERIAL_MAX_N ? LU_SERIAL : LU_GROUPED;
+// Columns per group: a smaller group wastes fewer updates beyond the shrinking row (a group's columns
+// all run at its first one's width), a larger one is less code and less shared memory.  B200, ms:
+// N = 6 (five-point FP64) 13.61 at 2, 13.66 at 3, 13.82 at 1, 13.88 at 6; N = 12 (gen-3v-4pt FP64)
+// 93.7 at 4, 95.3 at 3, 102.6 at 2 and 108.5 at 6; N = 30 FP64 115.4 at 10, 124.9 at 6, 131 at 15.
+__host__ __device__ constexpr int lu_group(int N) { return N <= 6 ? 2 : N <= 16 ? 4 : N <= 18 ? 6 : 10; }
+// stored pivot rows of a group that starts with rows of w entries: even stride (with the right-hand
+// side at entry w), so that the back substitution's diagonal reads fall into different banks
+__host__ __device__ constexpr int lu_row_stride(int w) { return (w + 2) & ~1; }
+// offset of column i's stored pivot row
+__host__ __device__ constexpr int lu_row_off(int N, int i) {
+  int off = 0;
+  for (int c = 0; c < N; c += lu_group(N)) {
+    const int w = N - c;
+    if (i < c + lu_group(N)) return off + (i - c) * lu_row_stride(w);
+    off += lu_group(N) * lu_row_stride(w);
+  }
+  return off;
+}
+// complex values of the per-sub-warp solve scratch sx: the pivot rows with their right-hand sides,
 // or, for the serial form, the whole system
-__host__ __device__ inline int lu_scratch_len(int N) {
-  return N <= GHC_LU_SERIAL_MAX_N ? N * (N + 1) : 2 * (N + 1);
+__host__ __device__ constexpr int lu_scratch_len(int N) {
+  return N <= GHC_LU_SERIAL_MAX_N ? N * (N + 1)
+                                  : lu_row_off(N, N - 1) + lu_row_stride(N - (N - 1) / lu_group(N) * lu_group(N));
 }
 
 // Pivot position of column i by the reference's rule (dev-cgesv-batched-small.cuh:54-65): the
@@ -451,182 +466,121 @@ __device__ __forceinline__ int pivot_redux3(R m, bool cand, int pos, int i) {
 template <int W>
 constexpr bool kPivotRedux3 = W == 16 || W == 32;
 
-// PivotRange: what one solve saw of its pivot magnitudes |U_ii| (|Re|+|Im|), in the oracle's
-// comparison order.  singular(): a zero pivot, unless column 0's magnitude was NaN (the oracle's
-// running minimum then stays NaN).  With SPAN (the mixed tracker's conditioning test) also the
-// smallest and largest magnitudes and whether any was NaN; without it only two flags stay live
-// across the LU.
+// PivotRange: what one solve saw of its pivot magnitudes |U_ii| (|Re|+|Im|).  singular(): a zero
+// pivot, unless column 0's magnitude was NaN (the oracle's running minimum then stays NaN).  With
+// SPAN (the mixed tracker's conditioning test) also the smallest and largest magnitudes and whether
+// any was NaN; without it only two flags stay live across the LU.
 template <typename R, bool SPAN>
 struct PivotRange {
-  R lo, hi;
-  bool nan, zero, nan0;
-  __device__ __forceinline__ void add(int i, R pm) {
-    if (i == 0) {
-      nan0 = pm != pm;
-      zero = pm == R(0);
-    } else {
-      zero = zero || pm == R(0);
-    }
+  R lo = R(__builtin_huge_val()), hi = R(0);
+  bool nan = false, zero = false, nan0 = false;
+  __device__ __forceinline__ void add(bool first, R pm) {
+    if (first) nan0 = pm != pm;
+    zero = zero || pm == R(0);
     if constexpr (SPAN) {
-      lo = (i == 0 || pm < lo) ? pm : lo;
-      hi = (i == 0 || pm > hi) ? pm : hi;
-      nan = (i != 0 && nan) || pm != pm;
+      lo = pm < lo ? pm : lo;
+      hi = pm > hi ? pm : hi;
+      nan = nan || pm != pm;
     }
   }
   __device__ __forceinline__ bool singular() const { return zero && !nan0; }
 };
 
+// returns this lane's component of the solution (lane l < N: component l)
 template <typename R, int N, int W, bool SPAN>
-__device__ __forceinline__ void lu_solve_unrolled(cx<R> (&A)[N], cx<R> b, int l, cx<R>* sx, cx<R>* sol,
+__device__ __forceinline__ cx<R> lu_solve_grouped(cx<R> (&A)[N], cx<R> b, int l, cx<R>* sx, cx<R>* sol,
                                                   PivotRange<R, SPAN>& rg) {
-  const bool live = l < N;
-  int pos = l;
-  static_for<0, N>([&](auto ic) {
-    constexpr int i = decltype(ic)::value;
-    cx<R>* px = sx + (i & 1) * (N + 1);
-    const R m = fabs(A[i].re) + fabs(A[i].im);
-    const bool cand = live && pos >= i;
-    int bp;
-    unsigned key = 0u, best = 0u;
-    if constexpr (kPivotRedux3<W>) {
-      bp = pivot_redux3<R, W>(m, cand, pos, i);
-    } else {
-      key = live ? pivot_key(m, pos, i) : 0u;
-      best = pivot_fast<R, W>(key);
-      bp = 31 - (int)(best & 31u);
-    }
-    if (live && pos == bp) {
-      static_for<i, N>([&](auto jc) { px[decltype(jc)::value] = A[decltype(jc)::value]; });
-      px[N] = b;
-    }
-    __syncwarp(kFull);
-    cx<R> p_i = px[i];
-    R pm = fabs(p_i.re) + fabs(p_i.im);
-    if (!kPivotRedux3<W> && __any_sync(kFull, cut_was_wrong(m, key, best, cand, pm))) {
-      bp = pivot_exact<R, W>(m, cand, pos, i);
-      __syncwarp(kFull);  // every lane has read the first choice
-      if (live && pos == bp) {
-        static_for<i, N>([&](auto jc) { px[decltype(jc)::value] = A[decltype(jc)::value]; });
-        px[N] = b;
+  constexpr int G = lu_group(N);
+  int pos = l < N ? l : -1;  // the row's position; -1: pivoted (or no row)
+  static_for<0, (N + G - 1) / G>([&](auto gc) {
+    constexpr int c0 = decltype(gc)::value * G, w = N - c0, n = w < G ? w : G;
+    cx<R>* px = sx + lu_row_off(N, c0);
+#pragma unroll 1
+    for (int i = c0; i < c0 + n; ++i, px += lu_row_stride(w)) {
+      const R m = fabs(A[0].re) + fabs(A[0].im);
+      const bool cand = pos >= i;
+      auto store = [&]() {
+        static_for<0, w>([&](auto jc) { px[decltype(jc)::value] = A[decltype(jc)::value]; });
+        px[w] = b;
+      };
+      int bp;
+      unsigned key = 0u, best = 0u;
+      if constexpr (kPivotRedux3<W>) {
+        bp = pivot_redux3<R, W>(m, cand, pos, i);
+      } else {
+        key = cand ? pivot_key(m, pos, i) : 0u;
+        best = pivot_fast<R, W>(key);
+        bp = 31 - (int)(best & 31u);
       }
+      if (pos == bp) store();
       __syncwarp(kFull);
-      p_i = px[i];
-      pm = fabs(p_i.re) + fabs(p_i.im);
-    }
-    const bool is_piv = live && (pos == bp);
-    if (live) {
-      if (pos == bp) pos = i;
-      else if (pos == i) pos = bp;
-    }
-    const bool zero = (pm == R(0));
-    rg.add(i, pm);
-    // (a zero pivot's reciprocal is NaN, as the oracle's c_rcp(0))
-    const cx<R> rc = c_rcp(p_i);
-    // the pivot row's reciprocal waits in the solution slot of its position until the back
-    // substitution (the slot is written there only after this lane has read it)
-    if (is_piv) sol[i] = rc;
-    // rows below the pivot take the update, the others keep their values
-    const bool upd = live && pos > i && !zero;
-    if (upd) {
-      A[i] = c_mul(A[i], rc);
-      static_for<i + 1, N>([&](auto jc) {
-        constexpr int j = decltype(jc)::value;
-        A[j] = c_fnma(A[i], px[j], A[j]);
-      });
-      b = c_fnma(A[i], px[N], b);
+      cx<R> p_i = px[0];
+      R pm = fabs(p_i.re) + fabs(p_i.im);
+      if (!kPivotRedux3<W> && __any_sync(kFull, cut_was_wrong(m, key, best, cand, pm))) {
+        bp = pivot_exact<R, W>(m, cand, pos, i);
+        __syncwarp(kFull);  // every lane has read the first choice
+        if (pos == bp) store();
+        __syncwarp(kFull);
+        p_i = px[0];
+        pm = fabs(p_i.re) + fabs(p_i.im);
+      }
+      rg.add(c0 == 0 && i == 0, pm);
+      // (a zero pivot's reciprocal is NaN, as the oracle's c_rcp(0))
+      const cx<R> rc = c_rcp(p_i);
+      if (pos == bp) {
+        sol[i] = rc;  // waits in the solution slot of its position until the back substitution
+        pos = -1;
+      } else if (pos == i) {
+        pos = bp;
+      }
+      const cx<R> f = c_mul(A[0], rc);
+      if (__any_sync(kFull, pm == R(0))) {  // rare: a path of the warp skips the column
+        const bool skip = pm == R(0);
+        static_for<0, w - 1>([&](auto jc) {
+          constexpr int j = decltype(jc)::value;
+          const cx<R> u = c_fnma(f, px[j + 1], A[j + 1]);
+          A[j] = skip ? A[j + 1] : u;
+        });
+        const cx<R> u = c_fnma(f, px[w], b);
+        b = skip ? b : u;
+      } else {
+        static_for<0, w - 1>([&](auto jc) {
+          constexpr int j = decltype(jc)::value;
+          A[j] = c_fnma(f, px[j + 1], A[j + 1]);
+        });
+        b = c_fnma(f, px[w], b);
+      }
     }
   });
-  static_for<0, N>([&](auto ic) {
-    constexpr int i = N - 1 - decltype(ic)::value;
-    if (live && pos == i) sol[i] = c_mul(b, sol[i]);
-    __syncwarp(kFull);
-    const cx<R> xi = sol[i];
-    if (live && pos < i) b = c_fnma(A[i], xi, b);
+  __syncwarp(kFull);  // the pivot rows and reciprocals are stored
+  // back substitution: lane l takes the pivot row of position l
+  const cx<R>* row = sx;
+  int w = N;
+  static_for<0, (N + G - 1) / G>([&](auto gc) {
+    constexpr int c0 = decltype(gc)::value * G;
+    if (l >= c0 && l < N) {
+      row = sx + lu_row_off(N, c0) + (l - c0) * lu_row_stride(N - c0);
+      w = N - c0;
+    }
   });
-  __syncwarp(kFull);
-}
-
-template <typename R, int N>
-__device__ __forceinline__ cx<R> pick(const cx<R> (&A)[N], int i) {
-  cx<R> a = A[0];
-#pragma unroll
-  for (int j = 1; j < N; ++j)
-    if (j == i) a = A[j];
-  return a;
-}
-
-template <typename R, int N, int W, bool SPAN>
-__device__ __forceinline__ void lu_solve_rolled(cx<R> (&A)[N], cx<R> b, int l, cx<R>* sx, cx<R>* sol,
-                                                PivotRange<R, SPAN>& rg) {
-  const bool live = l < N;
-  int pos = l;
-  cx<R> myrcp = mk(R(0), R(0));
-#pragma unroll 1
-  for (int i = 0; i < N; ++i) {
-    cx<R> ai = pick(A, i);
-    const R m = fabs(ai.re) + fabs(ai.im);
-    const bool cand = live && pos >= i;
-    const unsigned key = live ? pivot_key(m, pos, i) : 0u;
-    const unsigned best = pivot_fast<R, W>(key);
-    int bp = 31 - (int)(best & 31u);
-    if (live && pos == bp) {
-#pragma unroll
-      for (int j = 0; j < N; ++j)
-        if (j >= i) sx[j] = A[j];
-      sx[N] = b;
-    }
-    __syncwarp(kFull);
-    cx<R> p_i = sx[i];
-    R pm = fabs(p_i.re) + fabs(p_i.im);
-    if (__any_sync(kFull, cut_was_wrong(m, key, best, cand, pm))) {
-      bp = pivot_exact<R, W>(m, cand, pos, i);
-      __syncwarp(kFull);  // every lane has read the first choice
-      if (live && pos == bp) {
-#pragma unroll
-        for (int j = 0; j < N; ++j)
-          if (j >= i) sx[j] = A[j];
-        sx[N] = b;
-      }
-      __syncwarp(kFull);
-      p_i = sx[i];
-      pm = fabs(p_i.re) + fabs(p_i.im);
-    }
-    const bool is_piv = live && (pos == bp);
-    if (live) {
-      if (pos == bp) pos = i;
-      else if (pos == i) pos = bp;
-    }
-    const bool zero = (pm == R(0));
-    rg.add(i, pm);
-    const cx<R> rc = c_rcp(zero ? mk(R(0), R(0)) : p_i);
-    if (is_piv) myrcp = rc;
-    if (live && pos > i && !zero) {
-      ai = c_mul(ai, rc);
-#pragma unroll
-      for (int j = 0; j < N; ++j) {
-        if (j == i) A[j] = ai;
-        if (j > i) A[j] = c_fnma(ai, sx[j], A[j]);
-      }
-      b = c_fnma(ai, sx[N], b);
-    }
-    __syncwarp(kFull);
+  b = row[w];
+  const cx<R> rc = l < N ? sol[l] : mk(R(0), R(0));
+#pragma unroll 2
+  for (int i = N - 1; i > 0; --i) {
+    const cx<R> z = c_mul(b, rc);
+    const cx<R> xi = mk(__shfl_sync(kFull, z.re, i, W), __shfl_sync(kFull, z.im, i, W));
+    if (l < i) b = c_fnma(row[i - l], xi, b);
   }
-#pragma unroll 1
-  for (int i = N - 1; i >= 0; --i) {
-    if (live && pos == i) sol[i] = c_mul(b, myrcp);
-    __syncwarp(kFull);
-    const cx<R> xi = sol[i];
-    if (live && pos < i) b = c_fnma(pick(A, i), xi, b);
-  }
-  __syncwarp(kFull);
+  __syncwarp(kFull);  // the scratch may be written again
+  return c_mul(b, rc);
 }
 
 // The serial form: the oracle's elimination (rows at positions, strict-> scan from position i,
 // zero pivot skipping its column, back substitution by the stored reciprocals) run by every lane
-// on its own copy of the system; lane l leaves component l of the solution in sol[l].
+// on its own copy of the system; returns component l of the solution in lane l < N.
 template <typename R, int N, int W, bool SPAN>
-__device__ __forceinline__ void lu_solve_serial(cx<R> (&A)[N], cx<R> b, int l, cx<R>* sx, cx<R>* sol,
-                                                PivotRange<R, SPAN>& rg) {
+__device__ __forceinline__ cx<R> lu_solve_serial(cx<R> (&A)[N], cx<R> b, int l, cx<R>* sx,
+                                                 PivotRange<R, SPAN>& rg) {
   constexpr int C = N + 1;  // row length with the right-hand side
   if (l < N) {
     static_for<0, N>([&](auto jc) { sx[l * C + decltype(jc)::value] = A[decltype(jc)::value]; });
@@ -651,7 +605,7 @@ __device__ __forceinline__ void lu_solve_serial(cx<R> (&A)[N], cx<R> b, int l, c
         bp = j;
       }
     });
-    rg.add(i, best);
+    rg.add(i == 0, best);
     // the pivot row moves to position i, the row at position i to the pivot's position
     static_for<i + 1, N>([&](auto jc) {
       constexpr int j = decltype(jc)::value;
@@ -690,21 +644,19 @@ __device__ __forceinline__ void lu_solve_serial(cx<R> (&A)[N], cx<R> b, int l, c
   static_for<1, N>([&](auto jc) {
     if (l == decltype(jc)::value) mine = z[decltype(jc)::value];
   });
-  if (l < N) sol[l] = mine;
-  __syncwarp(kFull);
+  return mine;
 }
 
 template <typename R, int N, int W, bool SPAN>
-__device__ __forceinline__ void lu_solve(cx<R> (&A)[N], cx<R> b, int l, cx<R>* sx, cx<R>* sol,
-                                         PivotRange<R, SPAN>& rg) {
-  if constexpr (kLuForm<N> == LU_SERIAL) lu_solve_serial<R, N, W>(A, b, l, sx, sol, rg);
-  else if constexpr (kLuForm<N> == LU_ROLLED) lu_solve_rolled<R, N, W>(A, b, l, sx, sol, rg);
-  else lu_solve_unrolled<R, N, W>(A, b, l, sx, sol, rg);
+__device__ __forceinline__ cx<R> lu_solve(cx<R> (&A)[N], cx<R> b, int l, cx<R>* sx, cx<R>* sol,
+                                          PivotRange<R, SPAN>& rg) {
+  if constexpr (kLuForm<N> == LU_SERIAL) return lu_solve_serial<R, N, W>(A, b, l, sx, rg);
+  else return lu_solve_grouped<R, N, W>(A, b, l, sx, sol, rg);
 }
 template <typename R, int N, int W>
-__device__ __forceinline__ void lu_solve(cx<R> (&A)[N], cx<R> b, int l, cx<R>* sx, cx<R>* sol) {
+__device__ __forceinline__ cx<R> lu_solve(cx<R> (&A)[N], cx<R> b, int l, cx<R>* sx, cx<R>* sol) {
   PivotRange<R, false> rg;
-  lu_solve<R, N, W>(A, b, l, sx, sol, rg);
+  return lu_solve<R, N, W>(A, b, l, sx, sol, rg);
 }
 
 // xor-butterfly sum over the first NP lanes of the sub-warp (order = oracle tree_sum)
@@ -722,8 +674,8 @@ struct SubMem {
   unsigned char* coefA;  // c_k(t)   or p(t)     [Mc]
   unsigned char* coefB;  // c'_k(t)  or p1 - p0  [Mc]
   unsigned char* xs;     // track [N+1]
-  unsigned char* sx;     // solve scratch [lu_scratch_len(N)]: two pivot rows + rhs, or the whole system
-  unsigned char* sol;    // solution [N]
+  unsigned char* sx;     // solve scratch [lu_scratch_len(N)]: the pivot rows + rhs, or the whole system
+  unsigned char* sol;    // pivot reciprocals [N]
   unsigned char* state;  // per lane: RK base point x0 [W], RK accumulator [W] (state precision)
   unsigned char* scr;    // H_x row scratch [slots][W], null unless the evaluation is flat
   unsigned char* rec;    // the path's scalar state while the sub-warp evaluates and solves [kRecBytes]
@@ -778,12 +730,12 @@ __device__ __forceinline__ cx<R> eval_solve(const Tables& tb, const SubMem& sm, 
   eval_any<R, RL, N, W, KIND, S>(tb, sm, l, A, b, which);
   constexpr bool kSpan = !std::is_same<R, RL>::value;  // only the mixed tracker tests conditioning
   PivotRange<RL, kSpan> rg;
-  lu_solve<RL, N, W>(A, b, l, view<RL>(sm.sx), view<RL>(sm.sol), rg);
+  __syncwarp(kFull);  // the solve's scratch shares the row scratch's memory
+  const cx<RL> z = lu_solve<RL, N, W>(A, b, l, view<RL>(sm.sx), view<RL>(sm.sol), rg);
   if constexpr (kSpan) ill = cond_limit > 0.0 && (rg.nan || !(rg.hi <= (RL)cond_limit * rg.lo));
   else ill = false;
   sing = rg.singular();
-  const cx<RL> k = (l < N) ? view<RL>(sm.sol)[l] : mk(RL(0), RL(0));
-  return c_cast<R>(k);
+  return l < N ? c_cast<R>(z) : mk(R(0), R(0));
 }
 template <typename R, typename RL, int N, int W, int KIND, int S>
 __device__ __forceinline__ cx<R> eval_solve(const Tables& tb, const SubMem& sm, int l, int which) {
@@ -838,15 +790,13 @@ __host__ __device__ inline SubOffsets sub_offsets(int N, int Mc, int W, int slot
   off += (size_t)e * Mc;
   o.xs = off;
   off += (size_t)e * (N + 1);
-  o.sx = off;
-  off += (size_t)e * lu_scratch_len(N);
   o.sol = off;
   off += (size_t)e * N;
   if (mixed) off = align16(off);
   o.state = off;
   off += (size_t)es * 2 * W;
-  o.scr = off;
-  off += (size_t)e * slots * W;
+  o.sx = o.scr = off;
+  off += (size_t)e * (slots * W > lu_scratch_len(N) ? slots * W : lu_scratch_len(N));
   o.coefH = o.xsH = 0;
   if (mixed) {
     off = align16(off);
