@@ -106,31 +106,99 @@ __device__ __forceinline__ cx<R> c_cast(cx<S> a) {
 __device__ __forceinline__ double shfl_xor(double v, int off, int w) { return __shfl_xor_sync(kFull, v, off, w); }
 __device__ __forceinline__ float shfl_xor(float v, int off, int w) { return __shfl_xor_sync(kFull, v, off, w); }
 
-// compiled tables staged in shared memory
+// Compiled tables staged in shared memory.  The straight-line term shapes (NV >= 0 variable slots)
+// keep their terms there as packed words, decoded in about half the instructions of the compiled
+// 64-bit term words (the scale needs no integer conversion, the first variable's address is one
+// shift-add), for complex values of type R (B200: 5-point FP64 13.6 -> 13.2 ms, CY 95.4 -> 93.4,
+// gen-3v-4pt 93.8 -> 91.8, the mix 60.9 -> 57.3):
+//   lo  0.. 9  P2C coefficient index; PH: parameter index a (0..5) and b (6..11)
+//   lo 12..22  H_x, balanced walk: where the entry's sum goes (slot * W + row); third variable (12..16)
+//   lo 27..31  first variable
+//   hi  .. 8   second variable as a byte offset (5 bits from bit 4, complex double; 3, complex float)
+//   hi 13      H_x: the last term of its entry
+//   hi 14..31  the integer scale as R: the upper bits of the double's upper word, or of the float
+// The general shape (NV < 0) keeps the compiled words.
 struct Tables {
-  const uint64_t* hx_terms;
+  const uint2* hx_terms;
   const uint16_t* hx_off;
-  const uint64_t* ht_terms;
+  const uint2* ht_terms;
+  const uint2* ht_terms_hi;  // the terms packed for the state precision (mixed tracker's residual)
   const uint16_t* ht_off;
 };
+
+__device__ __forceinline__ uint64_t raw_word(uint2 w) { return (uint64_t)w.y << 32 | w.x; }
+template <typename R>
+constexpr unsigned kCxShift = sizeof(R) == 8 ? 4 : 3;  // log2 of a complex value's bytes
+
+template <typename R, int KIND, int NV>
+__device__ __forceinline__ uint2 pack_term(uint64_t w, int W) {
+  if (NV < 0) return make_uint2((unsigned)w, (unsigned)(w >> 32));
+  const unsigned s = sizeof(R) == 8 ? (unsigned)__double2hiint((double)term_scale(w))
+                                    : __float_as_uint((float)term_scale(w));
+  unsigned lo = KIND == KIND_P2C ? (unsigned)term_coef(w) : (unsigned)(term_pa(w) | term_pb(w) << 6);
+  unsigned hi = s & 0xffffc000u;
+  if (term_last(w)) hi |= 1u << 13;
+  lo |= (unsigned)term_var(w, 0) << 27;
+  if (NV >= 2) hi |= (unsigned)term_var(w, 1) << kCxShift<R>;
+  if (NV >= 3) lo |= (unsigned)term_var(w, 2) << 12;
+  else lo |= (unsigned)(term_dst_slot(w) * W + term_dst_row(w)) << 12;
+  return make_uint2(lo, hi);
+}
+template <int NV>
+__device__ __forceinline__ bool word_last(uint2 w) {
+  return NV < 0 ? term_last(raw_word(w)) : (w.y & (1u << 13)) != 0u;
+}
+template <int NV>
+__device__ __forceinline__ unsigned word_dst(uint2 w, int W) {
+  if (NV < 0) return (unsigned)(term_dst_slot(raw_word(w)) * W + term_dst_row(raw_word(w)));
+  return w.x >> 12 & 0x7ffu;
+}
+template <typename R, int NV>
+__device__ __forceinline__ R word_scale(uint2 w) {
+  if constexpr (NV < 0) return (R)term_scale(raw_word(w));
+  else if constexpr (sizeof(R) == 8) return __hiloint2double((int)(w.y & 0xffffc000u), 0);
+  else return __uint_as_float(w.y & 0xffffc000u);
+}
+template <typename R>
+__device__ __forceinline__ cx<R> at(const unsigned char* base, unsigned off) {
+  return *reinterpret_cast<const cx<R>*>(base + off);
+}
+// coefficient (P2C) or first / second parameter (PH) of a term, from an array of complex R
+template <typename R, int KIND, int NV>
+__device__ __forceinline__ cx<R> word_coef(uint2 w, const unsigned char* c) {
+  if (NV < 0) return at<R>(c, (unsigned)(KIND == KIND_P2C ? term_coef(raw_word(w)) : term_pa(raw_word(w))) << kCxShift<R>);
+  return at<R>(c, (w.x & (KIND == KIND_P2C ? 0x3ffu : 0x3fu)) << kCxShift<R>);
+}
+template <typename R, int NV>
+__device__ __forceinline__ cx<R> word_coef_b(uint2 w, const unsigned char* c) {
+  return at<R>(c, (NV < 0 ? (unsigned)term_pb(raw_word(w)) : w.x >> 6 & 0x3fu) << kCxShift<R>);
+}
 
 // acc += p * x[v0] * x[v1] ... over the term's variable slots (reference monomial term,
 // dev-eval-indxing-P3P.cuh:70-118; slot N is the constant 1).  Every term of a table has
 // the same number of slots: NV >= 0 fixes it at compile time (straight-line code), NV < 0
 // reads it from the word.
 template <typename R, int NV>
-__device__ __forceinline__ cx<R> acc_term(cx<R> acc, cx<R> p, uint64_t w, const cx<R>* xs) {
-  if constexpr (NV >= 0) {
-    if (NV == 0) return c_add(acc, p);
-#pragma unroll
-    for (int q = 0; q < NV - 1; ++q) p = c_mul(p, xs[term_var(w, q)]);
-    return c_fma(p, xs[term_var(w, NV - 1)], acc);
+__device__ __forceinline__ cx<R> acc_term(cx<R> acc, cx<R> p, uint2 w, const unsigned char* xs) {
+  static_assert(NV <= 3, "packed words hold three variables");
+  if constexpr (NV == 0) {
+    return c_add(acc, p);
+  } else if constexpr (NV > 0) {
+    const cx<R> x0 = at<R>(xs, w.x >> (27 - kCxShift<R>));
+    if constexpr (NV == 1) return c_fma(p, x0, acc);
+    p = c_mul(p, x0);
+    const cx<R> x1 = at<R>(xs, w.y & (31u << kCxShift<R>));
+    if constexpr (NV == 2) return c_fma(p, x1, acc);
+    p = c_mul(p, x1);
+    return c_fma(p, at<R>(xs, (w.x >> 12 & 31u) << kCxShift<R>), acc);
   } else {
-    const int nv = term_nv(w);
+    const uint64_t r = raw_word(w);
+    const cx<R>* x = reinterpret_cast<const cx<R>*>(xs);
+    const int nv = term_nv(r);
     if (nv == 0) return c_add(acc, p);
 #pragma unroll 1
-    for (int q = 0; q < nv - 1; ++q) p = c_mul(p, xs[term_var(w, q)]);
-    return c_fma(p, xs[term_var(w, nv - 1)], acc);
+    for (int q = 0; q < nv - 1; ++q) p = c_mul(p, x[term_var(r, q)]);
+    return c_fma(p, x[term_var(r, nv - 1)], acc);
   }
 }
 
@@ -179,11 +247,11 @@ __device__ __forceinline__ void coef_eval_ph(const double* __restrict__ ps, cons
 }
 
 // term value p (coefficient, or product of two homotopy parameters, times the integer scale)
-template <typename R, int KIND>
-__device__ __forceinline__ cx<R> term_coef_value(uint64_t w, const cx<R>* ca) {
-  if (KIND == KIND_P2C) return c_scale((R)term_scale(w), ca[term_coef(w)]);
-  const cx<R> p = c_scale((R)term_scale(w), ca[term_pa(w)]);
-  return c_mul(p, ca[term_pb(w)]);
+template <typename R, int KIND, int NV>
+__device__ __forceinline__ cx<R> term_coef_value(uint2 w, const unsigned char* ca) {
+  const cx<R> p = c_scale(word_scale<R, NV>(w), word_coef<R, KIND, NV>(w, ca));
+  if (KIND == KIND_P2C) return p;
+  return c_mul(p, word_coef_b<R, NV>(w, ca));
 }
 
 // Row r of H_x into A.
@@ -205,25 +273,32 @@ __device__ __forceinline__ cx<R> term_coef_value(uint64_t w, const cx<R>* ca) {
 template <int N>
 constexpr bool kFlatAlways = N > 16;
 
+// Term walks unrolled by 4: the loads of the next terms hide behind the arithmetic of the first
+// (5-point FP64, 12 warps a SM: 14.2 ms rolled, 13.4 by 2, 13.2 by 4); above 16 unknowns the H_t walk
+// only by 2 (30x30 FP64 113.3 against 118.9 ms).
+template <int N>
+constexpr int kUnrollHt = N > 16 ? 2 : 4;
+
 // Row r of H (which = 0) or of -H_t (which = 1) from the H_t term table, in precision R
 template <typename R, int N, int KIND, int NVT>
-__device__ __forceinline__ cx<R> eval_rhs(const Tables& tb, const cx<R>* ca, const cx<R>* cb, const cx<R>* xs, int r,
-                                          bool live, int which) {
+__device__ __forceinline__ cx<R> eval_rhs(const uint2* terms, const uint16_t* off, const unsigned char* ca,
+                                          const unsigned char* cb, const unsigned char* xs, int r, bool live,
+                                          int which) {
   cx<R> h = mk(R(0), R(0));
   if (live) {
-    const int len = tb.ht_off[r + 1] - tb.ht_off[r];
-    for (int k = 0; k < len; ++k) {
-      const uint64_t w = tb.ht_terms[k * N + r];
+    const uint2* wp = terms + r;
+    const int len = off[r + 1] - off[r];
+    const unsigned char* c0 = KIND == KIND_P2C && which ? cb : ca;
+#pragma unroll(kUnrollHt<N>)
+    for (int q = 0; q < len; ++q) {
+      const uint2 w = wp[q * N];
       cx<R> p;
-      if (KIND == KIND_P2C) {
-        p = c_scale((R)term_scale(w), which ? cb[term_coef(w)] : ca[term_coef(w)]);
-      } else if (which) {
-        const int a = term_pa(w), bb = term_pb(w);
-        const cx<R> u = c_fma(cb[bb], ca[a], c_mul(cb[a], ca[bb]));
-        p = c_scale((R)term_scale(w), u);
+      if (KIND == KIND_P2C || !which) {
+        p = term_coef_value<R, KIND, NVT>(w, c0);
       } else {
-        p = c_scale((R)term_scale(w), ca[term_pa(w)]);
-        p = c_mul(p, ca[term_pb(w)]);
+        const cx<R> u = c_fma(word_coef_b<R, NVT>(w, cb), word_coef<R, KIND, NVT>(w, ca),
+                              c_mul(word_coef<R, KIND, NVT>(w, cb), word_coef_b<R, NVT>(w, ca)));
+        p = c_scale(word_scale<R, NVT>(w), u);
       }
       h = acc_term<R, NVT>(h, p, w, xs);
     }
@@ -232,9 +307,15 @@ __device__ __forceinline__ cx<R> eval_rhs(const Tables& tb, const cx<R>* ca, con
 }
 
 template <typename R, int N, int W, int KIND, int NVX>
-__device__ __forceinline__ void eval_row(const Tables& tb, const cx<R>* ca, const cx<R>* xs, int r, bool live,
-                                         cx<R> (&A)[N], int walk, unsigned char* scr, unsigned nz) {
-  auto slot = [&](int k) -> cx<R>* { return view<R>(scr) + (k * W + r); };
+__device__ __forceinline__ void eval_row(const Tables& tb, const unsigned char* ca, const unsigned char* xs, int r,
+                                         bool live, cx<R> (&A)[N], int walk, unsigned char* scr, unsigned nz) {
+  // the row's k-th non-zero entry waits in slot k (W complex values each) until the row is read back
+  auto read_back = [&]() {
+    const cx<R>* sp = view<R>(scr) + r;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      A[i] = ((nz >> i) & 1u) ? sp[__popc(nz & ((1u << i) - 1u)) * W] : mk(R(0), R(0));
+  };
   const int lanes = balanced_walk_built(N) ? tb.hx_off[N * N + 1] : kNoLanes;
   const bool balanced = balanced_walk_built(N) && walk == 2 && lanes != kNoLanes;
   if (!kFlatAlways<N> && walk == 0) {
@@ -244,8 +325,8 @@ __device__ __forceinline__ void eval_row(const Tables& tb, const cx<R>* ca, cons
       if (live) {
         const int base = tb.hx_off[r * N], j0 = tb.hx_off[r * N + i], j1 = tb.hx_off[r * N + i + 1];
         for (int j = j0; j < j1; ++j) {
-          const uint64_t w = tb.hx_terms[(j - base) * N + r];
-          acc = acc_term<R, NVX>(acc, term_coef_value<R, KIND>(w, ca), w, xs);
+          const uint2 w = tb.hx_terms[(j - base) * N + r];
+          acc = acc_term<R, NVX>(acc, term_coef_value<R, KIND, NVX>(w, ca), w, xs);
         }
       }
       A[i] = acc;
@@ -253,39 +334,40 @@ __device__ __forceinline__ void eval_row(const Tables& tb, const cx<R>* ca, cons
   } else if (balanced) {
     // this lane's share of the entries (every lane of the sub-warp takes part); each finished
     // sum goes into the slot of its row, read back after the sub-warp synchronises
+    const uint2* wp = tb.hx_terms + lanes + r;
     const int len = tb.hx_off[N * N + 2 + r];
     cx<R> acc = mk(R(0), R(0));
+#pragma unroll 4
     for (int q = 0; q < len; ++q) {
-      const uint64_t w = tb.hx_terms[lanes + q * W + r];
-      acc = acc_term<R, NVX>(acc, term_coef_value<R, KIND>(w, ca), w, xs);
-      if (term_last(w)) {
-        view<R>(scr)[term_dst_slot(w) * W + term_dst_row(w)] = acc;
+      const uint2 w = wp[q * W];
+      acc = acc_term<R, NVX>(acc, term_coef_value<R, KIND, NVX>(w, ca), w, xs);
+      if (word_last<NVX>(w)) {
+        view<R>(scr)[word_dst<NVX>(w, W)] = acc;
         acc = mk(R(0), R(0));
       }
     }
     __syncwarp(kFull);  // other lanes wrote this row's slots
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-      A[i] = ((nz >> i) & 1u) ? *slot(__popc(nz & ((1u << i) - 1u))) : mk(R(0), R(0));
+    read_back();
   } else {
     if (live) {
+      const uint2* wp = tb.hx_terms + r;
       const int len = tb.hx_off[r * N + N] - tb.hx_off[r * N];
-      int k = 0;
+      cx<R>* sp = view<R>(scr) + r;
       cx<R> acc = mk(R(0), R(0));
+#pragma unroll 4
       for (int q = 0; q < len; ++q) {
-        const uint64_t w = tb.hx_terms[q * N + r];
-        acc = acc_term<R, NVX>(acc, term_coef_value<R, KIND>(w, ca), w, xs);
-        if (term_last(w)) {  // the entry's sum is complete
-          *slot(k++) = acc;
+        const uint2 w = wp[q * N];
+        acc = acc_term<R, NVX>(acc, term_coef_value<R, KIND, NVX>(w, ca), w, xs);
+        if (word_last<NVX>(w)) {  // the entry's sum is complete
+          *sp = acc;
+          sp += W;
           acc = mk(R(0), R(0));
         }
       }
     }
     // row-wise: this lane's own slots (each walk reads back inside its own branch: a read-back
     // shared by the walks after the branches cost hundreds of bytes of register spills)
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-      A[i] = ((nz >> i) & 1u) ? *slot(__popc(nz & ((1u << i) - 1u))) : mk(R(0), R(0));
+    read_back();
   }
 }
 
@@ -499,8 +581,19 @@ __device__ __forceinline__ cx<R> lu_solve_grouped(cx<R> (&A)[N], cx<R> b, int l,
     for (int i = c0; i < c0 + n; ++i, px += lu_row_stride(w)) {
       const R m = fabs(A[0].re) + fabs(A[0].im);
       const bool cand = pos >= i;
+      // The group's later columns have shorter rows; leaving their last entries out (uniformly) spares
+      // shared-memory traffic, which bounds FP64 up to 16 unknowns (gen-3v-4pt 91.9 -> 89.8 ms, CY
+      // 93.9 -> 91.9); in FP32 and at N = 30 the added branches cost more (mixed 39.5 -> 40.9,
+      // 30x30 112.9 -> 118.2).
+      constexpr bool kTrim = sizeof(R) == 8 && N > 6 && N <= 16;
+      const int t = i - c0;
+      auto has = [&](auto jc) {
+        return !kTrim || decltype(jc)::value + n <= w || decltype(jc)::value < w - t;
+      };
       auto store = [&]() {
-        static_for<0, w>([&](auto jc) { px[decltype(jc)::value] = A[decltype(jc)::value]; });
+        static_for<0, w>([&](auto jc) {
+          if (has(jc)) px[decltype(jc)::value] = A[decltype(jc)::value];
+        });
         px[w] = b;
       };
       int bp;
@@ -546,7 +639,7 @@ __device__ __forceinline__ cx<R> lu_solve_grouped(cx<R> (&A)[N], cx<R> b, int l,
       } else {
         static_for<0, w - 1>([&](auto jc) {
           constexpr int j = decltype(jc)::value;
-          A[j] = c_fnma(f, px[j + 1], A[j + 1]);
+          if (has(std::integral_constant<int, j + 1>{})) A[j] = c_fnma(f, px[j + 1], A[j + 1]);
         });
         b = c_fnma(f, px[w], b);
       }
@@ -677,7 +770,7 @@ struct SubMem {
   unsigned char* sx;     // solve scratch [lu_scratch_len(N)]: the pivot rows + rhs, or the whole system
   unsigned char* sol;    // pivot reciprocals [N]
   unsigned char* state;  // per lane: RK base point x0 [W], RK accumulator [W] (state precision)
-  unsigned char* scr;    // H_x row scratch [slots][W], null unless the evaluation is flat
+  unsigned char* scr;    // H_x row scratch [slots][W] of the flat walks, in the solve scratch's place
   unsigned char* rec;    // the path's scalar state while the sub-warp evaluates and solves [kRecBytes]
   unsigned char* coefH;  // mixed: c_k(t) or p(t) in state precision, for the residual H [Mc] (else null)
   unsigned char* xsH;    // mixed: the track in state precision [N+1] (else null)
@@ -704,18 +797,15 @@ __device__ __forceinline__ unsigned row_mask(const uint16_t* hx_off, int r) {
 template <typename R, typename RL, int N, int W, int KIND, int S>
 __device__ __forceinline__ void eval_any(const Tables& tb, const SubMem& sm, int l, cx<RL> (&A)[N], cx<RL>& b,
                                          int which) {
-  eval_row<RL, N, W, KIND, shape_nvx(S)>(tb, view<RL>(sm.coefA), view<RL>(sm.xs), l, l < N, A, sm.walk, sm.scr,
-                                         sm.nz);
+  eval_row<RL, N, W, KIND, shape_nvx(S)>(tb, sm.coefA, sm.xs, l, l < N, A, sm.walk, sm.scr, sm.nz);
   if constexpr (std::is_same<R, RL>::value) {
-    b = eval_rhs<RL, N, KIND, shape_nvt(S)>(tb, view<RL>(sm.coefA), view<RL>(sm.coefB), view<RL>(sm.xs), l, l < N,
-                                            which);
+    b = eval_rhs<RL, N, KIND, shape_nvt(S)>(tb.ht_terms, tb.ht_off, sm.coefA, sm.coefB, sm.xs, l, l < N, which);
   } else {
     if (which)
-      b = eval_rhs<RL, N, KIND, shape_nvt(S)>(tb, view<RL>(sm.coefA), view<RL>(sm.coefB), view<RL>(sm.xs), l,
-                                              l < N, 1);
+      b = eval_rhs<RL, N, KIND, shape_nvt(S)>(tb.ht_terms, tb.ht_off, sm.coefA, sm.coefB, sm.xs, l, l < N, 1);
     else
-      b = c_cast<RL>(eval_rhs<R, N, KIND, shape_nvt(S)>(tb, view<R>(sm.coefH), view<R>(sm.coefH), view<R>(sm.xsH),
-                                                        l, l < N, 0));
+      b = c_cast<RL>(eval_rhs<R, N, KIND, shape_nvt(S)>(tb.ht_terms_hi, tb.ht_off, sm.coefH, sm.coefH, sm.xsH, l,
+                                                        l < N, 0));
   }
 }
 
@@ -743,16 +833,20 @@ __device__ __forceinline__ cx<R> eval_solve(const Tables& tb, const SubMem& sm, 
   return eval_solve<R, RL, N, W, KIND, S>(tb, sm, l, which, 0.0, ill, sing);
 }
 
-// the track into shared memory: in RL for H_x and H_t, and (mixed) in R for the residual
+// the track into shared memory: in RL for H_x and H_t, and (mixed) in R for the residual; its last
+// slot, the constant 1 of the term tables, is written once (write_one)
 template <typename R, typename RL, int N>
 __device__ __forceinline__ void write_track(const SubMem& sm, int l, cx<R> x) {
-  cx<RL>* xs = view<RL>(sm.xs);
-  if (l < N) xs[l] = c_cast<RL>(x);
-  if (l == 0) xs[N] = mk(RL(1), RL(0));
-  if constexpr (!std::is_same<R, RL>::value) {
-    cx<R>* xh = view<R>(sm.xsH);
-    if (l < N) xh[l] = x;
-    if (l == 0) xh[N] = mk(R(1), R(0));
+  if (l < N) {
+    view<RL>(sm.xs)[l] = c_cast<RL>(x);
+    if constexpr (!std::is_same<R, RL>::value) view<R>(sm.xsH)[l] = x;
+  }
+}
+template <typename R, typename RL, int N>
+__device__ __forceinline__ void write_one(const SubMem& sm, int l) {
+  if (l == 0) {
+    view<RL>(sm.xs)[N] = mk(RL(1), RL(0));
+    if constexpr (!std::is_same<R, RL>::value) view<R>(sm.xsH)[N] = mk(R(1), R(0));
   }
 }
 
@@ -770,13 +864,16 @@ __device__ __forceinline__ void coef_eval(const TrackParams& p, const SubMem& sm
 
 // byte sizes of the shared-memory layout
 __host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
-__host__ __device__ inline size_t tables_bytes(int N, int n_hx, int n_ht) {
-  return align16(8 * (size_t)(n_hx + n_ht) + 2 * (size_t)(hx_off_len(N) + N + 1));
+__host__ __device__ inline size_t tables_bytes(int N, int n_hx, int n_ht, bool mixed) {
+  return align16(8 * ((size_t)n_hx + (mixed ? 2 : 1) * (size_t)n_ht) + 2 * (size_t)(hx_off_len(N) + N + 1));
 }
 // Per sub-warp: the path record [kRecBytes], then, in complex values of e bytes (linear-algebra
-// precision): coefficient buffers [2 Mc], track [N+1], solve scratch [lu_scratch_len(N)], solution [N]; the
-// lane state [2 W] in complex values of es bytes (state precision); scratch slots [slots W] (flat);
-// and, when es != e (mixed), the state-precision coefficients [Mc] and track [N+1].
+// precision): track [N+1], pivot reciprocals [N]; the lane state [2 W] and, when es != e (mixed), the
+// state-precision track [N+1] in complex values of es bytes (state precision); the row scratch
+// [slots W] (flat) in the same place as the solve scratch [lu_scratch_len(N)]; the coefficient buffers
+// [2 Mc] and, mixed, the state-precision coefficients [Mc].  What the problem's tables do not size
+// comes first, so its offsets are constants of the kernel.  An odd multiple of 16 bytes: equal places
+// of two sub-warps never fall into the same banks.
 struct SubOffsets {
   size_t coefA, coefB, xs, sx, sol, state, scr, coefH, xsH, bytes;
 };
@@ -784,28 +881,30 @@ __host__ __device__ inline SubOffsets sub_offsets(int N, int Mc, int W, int slot
   const bool mixed = es != e;
   SubOffsets o;
   size_t off = kRecBytes;
+  o.xs = off;
+  off += (size_t)e * (N + 1);
+  o.sol = off;
+  off = align16(off + (size_t)e * N);
+  o.state = off;
+  off += (size_t)es * 2 * W;
+  o.xsH = 0;
+  if (mixed) {
+    o.xsH = off;
+    off += (size_t)es * (N + 1);
+  }
+  o.sx = o.scr = off;
+  off += (size_t)e * (slots * W > lu_scratch_len(N) ? slots * W : lu_scratch_len(N));
   o.coefA = off;
   off += (size_t)e * Mc;
   o.coefB = off;
   off += (size_t)e * Mc;
-  o.xs = off;
-  off += (size_t)e * (N + 1);
-  o.sol = off;
-  off += (size_t)e * N;
-  if (mixed) off = align16(off);
-  o.state = off;
-  off += (size_t)es * 2 * W;
-  o.sx = o.scr = off;
-  off += (size_t)e * (slots * W > lu_scratch_len(N) ? slots * W : lu_scratch_len(N));
-  o.coefH = o.xsH = 0;
+  o.coefH = 0;
   if (mixed) {
     off = align16(off);
     o.coefH = off;
     off += (size_t)es * Mc;
-    o.xsH = off;
-    off += (size_t)es * (N + 1);
   }
-  o.bytes = kRecBytes + align16(off - kRecBytes);
+  o.bytes = align16(off) | 16;
   return o;
 }
 __host__ __device__ inline size_t sub_bytes(int N, int Mc, int W, int slots, int e, int es) {
@@ -822,7 +921,7 @@ __device__ __forceinline__ SubMem sub_layout(unsigned char* base, int N, int Mc,
   sm.sx = base + o.sx;
   sm.sol = base + o.sol;
   sm.state = base + o.state;
-  sm.scr = flat ? base + o.scr : nullptr;
+  sm.scr = base + o.scr;
   const bool mixed = !std::is_same<R, RL>::value;
   sm.coefH = mixed ? base + o.coefH : nullptr;
   sm.xsH = mixed ? base + o.xsH : nullptr;
@@ -861,15 +960,22 @@ constexpr int track_min_blocks() {
                                     : (N <= 8 ? 10 : N <= 12 ? 8 : N <= 18 ? 5 : 4));
 }
 
+template <typename R, typename RL, int N, int KIND, int S>
 __device__ __forceinline__ Tables stage_tables(unsigned char* smem, const uint64_t* g_hx, const uint16_t* g_hxo,
-                                               const uint64_t* g_ht, const uint16_t* g_hto, int N, int n_hx,
-                                               int n_ht) {
-  uint64_t* s_hx = reinterpret_cast<uint64_t*>(smem);
-  uint64_t* s_ht = s_hx + n_hx;
-  uint16_t* s_hxo = reinterpret_cast<uint16_t*>(s_ht + n_ht);
+                                               const uint64_t* g_ht, const uint16_t* g_hto, int n_hx, int n_ht) {
+  constexpr bool mixed = !std::is_same<R, RL>::value;
+  constexpr int W = subwarp_width(N), NVX = shape_nvx(S), NVT = shape_nvt(S);
+  uint2* s_hx = reinterpret_cast<uint2*>(smem);
+  uint2* s_ht = s_hx + n_hx;
+  uint2* s_hth = mixed ? s_ht + n_ht : s_ht;
+  uint16_t* s_hxo = reinterpret_cast<uint16_t*>(s_hth + n_ht);
   uint16_t* s_hto = s_hxo + hx_off_len(N);
-  for (int i = threadIdx.x; i < n_hx; i += blockDim.x) s_hx[i] = __ldg(g_hx + i);
-  for (int i = threadIdx.x; i < n_ht; i += blockDim.x) s_ht[i] = __ldg(g_ht + i);
+  for (int i = threadIdx.x; i < n_hx; i += blockDim.x) s_hx[i] = pack_term<RL, KIND, NVX>(__ldg(g_hx + i), W);
+  for (int i = threadIdx.x; i < n_ht; i += blockDim.x) {
+    const uint64_t w = __ldg(g_ht + i);
+    s_ht[i] = pack_term<RL, KIND, NVT>(w, W);
+    if constexpr (mixed) s_hth[i] = pack_term<R, KIND, NVT>(w, W);
+  }
   for (int i = threadIdx.x; i < hx_off_len(N); i += blockDim.x) s_hxo[i] = __ldg(g_hxo + i);
   for (int i = threadIdx.x; i < N + 1; i += blockDim.x) s_hto[i] = __ldg(g_hto + i);
   __syncthreads();
@@ -877,6 +983,7 @@ __device__ __forceinline__ Tables stage_tables(unsigned char* smem, const uint64
   t.hx_terms = s_hx;
   t.hx_off = s_hxo;
   t.ht_terms = s_ht;
+  t.ht_terms_hi = s_hth;
   t.ht_off = s_hto;
   return t;
 }
@@ -926,7 +1033,8 @@ constexpr int track_block() {
 template <typename R, typename RL, int N, int W, int KIND, int S, int WK>
 __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* smem, long long cta, long long n_cta,
                                            bool visitor) {
-  const Tables tb = stage_tables(smem, p.hx_terms, p.hx_off, p.ht_terms, p.ht_off, N, p.n_hx_terms, p.n_ht_terms);
+  const Tables tb = stage_tables<R, RL, N, KIND, S>(smem, p.hx_terms, p.hx_off, p.ht_terms, p.ht_off, p.n_hx_terms,
+                                                    p.n_ht_terms);
 
   const int lane = threadIdx.x & 31;
   const int l = lane % W;
@@ -934,12 +1042,13 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const int walk = WK >= 0 ? WK : ((kFlatAlways<N> && p.flat_eval == 0) ? 1 : p.flat_eval);
   const bool flat = walk != 0;
-  SubMem sm = sub_layout<R, RL>(smem + tables_bytes(N, p.n_hx_terms, p.n_ht_terms) +
+  SubMem sm = sub_layout<R, RL>(smem + tables_bytes(N, p.n_hx_terms, p.n_ht_terms, !std::is_same<R, RL>::value) +
                                     (size_t)g * sub_bytes(N, Mc, W, flat ? p.scr_slots : 0, (int)sizeof(cx<RL>),
                                                           (int)sizeof(cx<R>)),
                                 N, Mc, W, p.scr_slots, flat);
   sm.nz = row_mask<N>(tb.hx_off, l);
   sm.walk = walk;
+  write_one<R, RL, N>(sm, l);
   // this lane's RK base point x0 and accumulator sols live in shared memory (register relief)
   cx<R>& x0 = view<R>(sm.state)[l];
   cx<R>& sols = view<R>(sm.state)[W + l];
@@ -1234,18 +1343,20 @@ __global__ void __launch_bounds__(GHC_BLOCK(N, R, RL, V), GHC_MINB(N, R, RL, V))
 template <int N, int W, int KIND, int S>
 __global__ void __launch_bounds__(128) polish_kernel(const PolishParams p) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const Tables tb = stage_tables(smem, p.hx_terms, p.hx_off, p.ht_terms, p.ht_off, N, p.n_hx_terms, p.n_ht_terms);
+  const Tables tb = stage_tables<double, double, N, KIND, S>(smem, p.hx_terms, p.hx_off, p.ht_terms, p.ht_off,
+                                                             p.n_hx_terms, p.n_ht_terms);
   const int lane = threadIdx.x & 31;
   const int l = lane % W;
   const int g = threadIdx.x / W;
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const int walk = (kFlatAlways<N> && p.flat_eval == 0) ? 1 : p.flat_eval;
   const bool flat = walk != 0;
-  SubMem sm = sub_layout<double, double>(smem + tables_bytes(N, p.n_hx_terms, p.n_ht_terms) +
+  SubMem sm = sub_layout<double, double>(smem + tables_bytes(N, p.n_hx_terms, p.n_ht_terms, false) +
                                              (size_t)g * sub_bytes(N, Mc, W, flat ? p.scr_slots : 0, 16, 16),
                                          N, Mc, W, p.scr_slots, flat);
   sm.nz = row_mask<N>(tb.hx_off, l);
   sm.walk = walk;
+  write_one<double, double, N>(sm, l);
   const int subs_per_cta = blockDim.x / W;
   const int leader = lane - l;
   for (long long item0 = (long long)blockIdx.x * subs_per_cta; item0 < p.n_items;

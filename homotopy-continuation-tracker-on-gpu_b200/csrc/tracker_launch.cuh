@@ -34,7 +34,7 @@ int launch_track_w(const TrackParams& p, cudaStream_t s, int n_sm) {
   auto kern = dev::track_kernel<R, RL, N, W, KIND, V, S, WK>;
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const int slots = (dev::kFlatAlways<N> || p.flat_eval) ? p.scr_slots : 0;
-  const size_t tables = dev::tables_bytes(N, p.n_hx_terms, p.n_ht_terms);
+  const size_t tables = dev::tables_bytes(N, p.n_hx_terms, p.n_ht_terms, !std::is_same<R, RL>::value);
   const size_t per_sub = dev::sub_bytes(N, Mc, W, slots, 2 * (int)sizeof(RL), 2 * (int)sizeof(R));
   const int block = block_threads(tables, per_sub, W, GHC_BLOCK(N, R, RL, V));
   if (block == 0) return -24;
@@ -117,7 +117,7 @@ int launch_polish_s(const PolishParams& p, cudaStream_t s) {
   auto kern = dev::polish_kernel<N, W, KIND, S>;
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const int slots = (dev::kFlatAlways<N> || p.flat_eval) ? p.scr_slots : 0;
-  const size_t tables = dev::tables_bytes(N, p.n_hx_terms, p.n_ht_terms);
+  const size_t tables = dev::tables_bytes(N, p.n_hx_terms, p.n_ht_terms, false);
   const size_t per_sub = dev::sub_bytes(N, Mc, W, slots, 16, 16);
   const int block = block_threads(tables, per_sub, W);
   if (block == 0) return -24;
