@@ -68,6 +68,7 @@ TrackParams base_params(const Problem& pb) {
   p.incr = pb.incr;
   p.n_hx_terms = (int)pb.hx_terms.size();
   p.n_ht_terms = (int)pb.ht_terms.size();
+  p.n_hx_rows = row_words(pb.hx_off.data(), pb.N, p.n_hx_terms);
   p.hx_terms = pb.dev.hx_terms;
   p.hx_off = pb.dev.hx_off;
   p.ht_terms = pb.dev.ht_terms;
@@ -92,6 +93,7 @@ PolishParams polish_params(const TrackParams& t, double* endpoints, const uint8_
   q.K = t.K;
   q.n_hx_terms = t.n_hx_terms;
   q.n_ht_terms = t.n_ht_terms;
+  q.n_hx_rows = t.n_hx_rows;
   q.flat_eval = t.flat_eval;
   q.scr_slots = t.scr_slots;
   q.shape = t.shape;
@@ -246,6 +248,7 @@ int dropin_tables(Problem& pb, const int* d_hx, const int* d_ht, TrackParams& p,
   p.ht_off = (const uint16_t*)c.dev[3];
   p.n_hx_terms = (int)c.hx_terms.size();
   p.n_ht_terms = (int)c.ht_terms.size();
+  p.n_hx_rows = row_words(c.hx_off.data(), pb.N, p.n_hx_terms);
   p.flat_eval = flat_eval_pays(c.hx_off.data(), pb.N);  // the caller's own tables: their own walk
   p.scr_slots = row_nonzeros_max(c.hx_off.data(), pb.N);
   return GHC_OK;

@@ -84,6 +84,13 @@ inline int row_nonzeros_max(const uint16_t* hx_off, int N) {
   return most;
 }
 
+// words of the row-interleaved section of the compiled H_x terms (n_hx words in all)
+inline int row_words(const uint16_t* hx_off, int N, int n_hx) {
+  return hx_off[N * N + 1] == kNoLanes ? n_hx : hx_off[N * N + 1];
+}
+// words that a CTA stages for a walk: only the section that the walk reads
+GHC_HD inline int staged_words(int walk, int n_hx, int n_rows) { return walk == 2 && n_rows < n_hx ? n_hx - n_rows : n_rows; }
+
 inline int flat_eval_pays(const uint16_t* hx_off, int N) {
   int longest = 0, per_entry = 0, walk = 1;
   for (int r = 0; r < N; ++r) {
@@ -131,6 +138,7 @@ struct TrackParams {
   int kind, N, P, M, K;
   int max_steps, max_corr, incr;
   int n_hx_terms, n_ht_terms;
+  int n_hx_rows;              // words of the row-interleaved H_x section (the balanced walk's follow)
   int flat_eval;              // H_x walk: 0 entry-wise, 1 row-wise, 2 balanced (flat_eval_pays() or the autotuner)
   int shape;                  // eval_shape_of() of the problem
   int scr_slots;              // row_nonzeros_max() of the tables
@@ -192,7 +200,7 @@ struct TrackParams {
 
 struct PolishParams {
   int kind, N, P, M, K;
-  int n_hx_terms, n_ht_terms;
+  int n_hx_terms, n_ht_terms, n_hx_rows;
   int flat_eval, scr_slots, shape;
   const uint64_t* hx_terms;
   const uint16_t* hx_off;

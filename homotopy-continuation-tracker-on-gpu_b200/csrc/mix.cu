@@ -95,7 +95,7 @@ size_t slot_smem(const TrackParams& p) {
   const int Mc = (SL::KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const int walk = SL::WK >= 0 ? SL::WK : ((dev::kFlatAlways<SL::N> && p.flat_eval == 0) ? 1 : p.flat_eval);
   const int slots = walk ? p.scr_slots : 0;
-  return dev::tables_bytes(SL::N, p.n_hx_terms, p.n_ht_terms, false) +
+  return dev::tables_bytes(SL::N, staged_words(walk, p.n_hx_terms, p.n_hx_rows), p.n_ht_terms, false) +
          (size_t)(kMixBlock / SL::W) * dev::sub_bytes(SL::N, Mc, SL::W, slots, 16, 16);
 }
 

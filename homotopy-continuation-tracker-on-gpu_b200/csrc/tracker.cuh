@@ -334,7 +334,7 @@ __device__ __forceinline__ void eval_row(const Tables& tb, const unsigned char* 
   } else if (balanced) {
     // this lane's share of the entries (every lane of the sub-warp takes part); each finished
     // sum goes into the slot of its row, read back after the sub-warp synchronises
-    const uint2* wp = tb.hx_terms + lanes + r;
+    const uint2* wp = tb.hx_terms + r;  // (the staged section is the balanced one)
     const int len = tb.hx_off[N * N + 2 + r];
     cx<R> acc = mk(R(0), R(0));
 #pragma unroll 4
@@ -940,32 +940,34 @@ __device__ __forceinline__ cx<R> load_cx(const void* base, bool f64, long long i
   return mk((R)f[0], (R)f[1]);
 }
 
-// CTAs per SM the tracker asks the register allocator for: the row of H_x (N
-// complex values) dominates the registers, so small systems afford more.  Two
-// compiled variants per size and precision; the autotuner (ghc_autotune) picks
-// one per problem.  Variant 0 is the best of B200 sweeps over the shipped
-// problems (512 hypotheses, autotuning off, 3..7 CTAs): FP64 N = 3 at 6 (at 8
-// the 64 registers spill), N = 6 flat within noise, N = 12 at 5 (generalized
-// 3-view 5360 vs 5326 hyp/s at 4, uncalibrated trifocal 1376 vs 1348; 6 and 7
-// spill), N = 30 at 3 (406 vs 397 at 4); FP32 N = 12 at 7, N = 30 at 5 (577
-// vs 552 at 3).  Variant 1 is the runner-up budget.  The mixed tracker (FP64 state, FP32
-// linear algebra) holds the row in FP32 and asks for about the FP32 budget.
+// CTAs of 128 threads per SM the tracker asks the register allocator for: the row of H_x (N complex
+// values) dominates the registers, so small systems afford more.  Two compiled variants per size and
+// precision; the autotuner (ghc_autotune) picks one per problem.  Variant 0 is the best of B200 sweeps
+// (autotuning off, 3..8 CTAs, ms): FP64 N = 3 (20,000 hypotheses) 2.14 at 6, 2.13 at 7, 2.26 at 4;
+// N = 6 (2,048) 12.4 at 4, 13.1 at 3, 12.8 at 6; N = 12 (gen-3v-4pt, 512) 92.1 at 5, 94.5 at 4, 101 at
+// 6; N = 30 (48) 113 at 3, 189 at 4 (spills).  FP32 N = 6 (1,000) 6.00 at 6, 6.11 at 8; N = 12 (200)
+// 111.9 at 6, 113.0 at 5, 118.4 at 7; N = 30 72.6 at 4, 74.8 at 5, 79.1 at 3.  The mixed tracker (FP64
+// state, FP32 linear algebra) N = 12 (251) 38.8 at 6, 38.7 at 5, 40.9 at 7; N = 30 73.3 at 4, 74.7 at
+// 3, 158 at 5.  Variant 1 is the runner-up budget.
 template <int N, typename R, typename RL, int V>
 constexpr int track_min_blocks() {
   return !std::is_same<R, RL>::value
              ? (V == 0 ? (N <= 8 ? 6 : N <= 12 ? 6 : N <= 18 ? 4 : 4) : (N <= 8 ? 8 : N <= 12 ? 5 : N <= 18 ? 5 : 3))
          : V == 0 ? (sizeof(R) == 8 ? (N <= 4 ? 6 : N <= 8 ? 4 : N <= 12 ? 5 : 3)
-                                    : (N <= 8 ? 8 : N <= 12 ? 7 : N <= 18 ? 4 : 5))
+                                    : (N <= 4 ? 8 : N <= 12 ? 6 : 4))
                   : (sizeof(R) == 8 ? (N <= 4 ? 8 : N <= 8 ? 6 : N <= 12 ? 4 : N <= 18 ? 4 : 2)
-                                    : (N <= 8 ? 10 : N <= 12 ? 8 : N <= 18 ? 5 : 4));
+                                    : (N <= 4 ? 10 : N <= 8 ? 8 : 5));
 }
 
 template <typename R, typename RL, int N, int KIND, int S>
 __device__ __forceinline__ Tables stage_tables(unsigned char* smem, const uint64_t* g_hx, const uint16_t* g_hxo,
-                                               const uint64_t* g_ht, const uint16_t* g_hto, int n_hx, int n_ht) {
+                                               const uint64_t* g_ht, const uint16_t* g_hto, int n_hx, int n_rows,
+                                               int n_ht, int walk) {
   constexpr bool mixed = !std::is_same<R, RL>::value;
   constexpr int W = subwarp_width(N), NVX = shape_nvx(S), NVT = shape_nvt(S);
   uint2* s_hx = reinterpret_cast<uint2*>(smem);
+  if (walk == 2 && n_rows < n_hx) g_hx += n_rows;
+  n_hx = staged_words(walk, n_hx, n_rows);
   uint2* s_ht = s_hx + n_hx;
   uint2* s_hth = mixed ? s_ht + n_ht : s_ht;
   uint16_t* s_hxo = reinterpret_cast<uint16_t*>(s_hth + n_ht);
@@ -1006,22 +1008,18 @@ __device__ __forceinline__ Tables stage_tables(unsigned char* smem, const uint64
 // A resuming launch (resume = 1) starts every item from track_in at t_in[i]
 // with step dt_in[i] and the step / corrector counts already in steps / corr.
 // -------------------------------------------------------------------------------------------------
-#ifdef GHC_TRACK_MIN_BLOCKS
-#define GHC_MINB(N, R, RL, V) GHC_TRACK_MIN_BLOCKS
-#else
-#define GHC_MINB(N, R, RL, V) ::ghc::dev::track_min_blocks<N, R, RL, V>()
-#endif
-// Threads per CTA of a tracker instantiation (the launch may still halve it when the per-sub-warp
-// shared memory does not fit).  128 everywhere by default.
+// Most threads per CTA of a tracker instantiation.  Where the coefficient buffers of a path, not the
+// registers, limit the paths on an SM (FP64 at 5 to 8 unknowns: 2.4 of 3.8 KB a path for the 75
+// coefficients of the five-point problem), the launch may use CTAs of up to 256 threads: one copy of
+// the tables serves more paths, and what shared memory remains is handed out in finer steps.
 template <int N, typename R, typename RL, int V>
 constexpr int track_block() {
-  return 128;
+  return track_min_blocks<N, R, RL, V>() % 2 == 0 && N > 4 && N <= 8 ? 256 : 128;
 }
-#ifdef GHC_TRACK_BLOCK
-#define GHC_BLOCK(N, R, RL, V) GHC_TRACK_BLOCK
-#else
-#define GHC_BLOCK(N, R, RL, V) ::ghc::dev::track_block<N, R, RL, V>()
-#endif
+template <int N, typename R, typename RL, int V>
+constexpr int track_ctas() {
+  return track_min_blocks<N, R, RL, V>() * 128 / track_block<N, R, RL, V>();
+}
 // WK >= 0: the H_x walk is fixed at compile time (only that walk's code is in the kernel, which
 // spares the register allocator the other walk's read-back: above 16 unknowns, where the row fills
 // most of the registers); WK < 0: chosen at run time from p.flat_eval.
@@ -1033,16 +1031,17 @@ constexpr int track_block() {
 template <typename R, typename RL, int N, int W, int KIND, int S, int WK>
 __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* smem, long long cta, long long n_cta,
                                            bool visitor) {
+  const int walk = WK >= 0 ? WK : ((kFlatAlways<N> && p.flat_eval == 0) ? 1 : p.flat_eval);
+  const int n_hx = staged_words(walk, p.n_hx_terms, p.n_hx_rows);
   const Tables tb = stage_tables<R, RL, N, KIND, S>(smem, p.hx_terms, p.hx_off, p.ht_terms, p.ht_off, p.n_hx_terms,
-                                                    p.n_ht_terms);
+                                                    p.n_hx_rows, p.n_ht_terms, walk);
 
   const int lane = threadIdx.x & 31;
   const int l = lane % W;
   const int g = threadIdx.x / W;
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
-  const int walk = WK >= 0 ? WK : ((kFlatAlways<N> && p.flat_eval == 0) ? 1 : p.flat_eval);
   const bool flat = walk != 0;
-  SubMem sm = sub_layout<R, RL>(smem + tables_bytes(N, p.n_hx_terms, p.n_ht_terms, !std::is_same<R, RL>::value) +
+  SubMem sm = sub_layout<R, RL>(smem + tables_bytes(N, n_hx, p.n_ht_terms, !std::is_same<R, RL>::value) +
                                     (size_t)g * sub_bytes(N, Mc, W, flat ? p.scr_slots : 0, (int)sizeof(cx<RL>),
                                                           (int)sizeof(cx<R>)),
                                 N, Mc, W, p.scr_slots, flat);
@@ -1332,7 +1331,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
 }
 
 template <typename R, typename RL, int N, int W, int KIND, int V, int S, int WK>
-__global__ void __launch_bounds__(GHC_BLOCK(N, R, RL, V), GHC_MINB(N, R, RL, V)) track_kernel(const TrackParams p) {
+__global__ void __launch_bounds__((track_block<N, R, RL, V>()), (track_ctas<N, R, RL, V>())) track_kernel(const TrackParams p) {
   extern __shared__ __align__(16) unsigned char smem[];
   track_body<R, RL, N, W, KIND, S, WK>(p, smem, blockIdx.x, gridDim.x, false);
 }
@@ -1343,15 +1342,16 @@ __global__ void __launch_bounds__(GHC_BLOCK(N, R, RL, V), GHC_MINB(N, R, RL, V))
 template <int N, int W, int KIND, int S>
 __global__ void __launch_bounds__(128) polish_kernel(const PolishParams p) {
   extern __shared__ __align__(16) unsigned char smem[];
+  const int walk = (kFlatAlways<N> && p.flat_eval == 0) ? 1 : p.flat_eval;
+  const int n_hx = staged_words(walk, p.n_hx_terms, p.n_hx_rows);
   const Tables tb = stage_tables<double, double, N, KIND, S>(smem, p.hx_terms, p.hx_off, p.ht_terms, p.ht_off,
-                                                             p.n_hx_terms, p.n_ht_terms);
+                                                             p.n_hx_terms, p.n_hx_rows, p.n_ht_terms, walk);
   const int lane = threadIdx.x & 31;
   const int l = lane % W;
   const int g = threadIdx.x / W;
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
-  const int walk = (kFlatAlways<N> && p.flat_eval == 0) ? 1 : p.flat_eval;
   const bool flat = walk != 0;
-  SubMem sm = sub_layout<double, double>(smem + tables_bytes(N, p.n_hx_terms, p.n_ht_terms, false) +
+  SubMem sm = sub_layout<double, double>(smem + tables_bytes(N, n_hx, p.n_ht_terms, false) +
                                              (size_t)g * sub_bytes(N, Mc, W, flat ? p.scr_slots : 0, 16, 16),
                                          N, Mc, W, p.scr_slots, flat);
   sm.nz = row_mask<N>(tb.hx_off, l);

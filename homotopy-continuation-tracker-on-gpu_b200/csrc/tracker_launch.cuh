@@ -15,7 +15,7 @@ constexpr int kBlock = 128;
 // Threads per CTA: 128, or fewer (64, 32) when that many sub-warps' shared memory (per-sub-warp
 // coefficient buffers grow with the problem's coefficient count: 565 complex values x 2 for the
 // generalized 3-view 6-line problem) exceeds what one CTA may use.  0: does not fit at all.
-inline int block_threads(size_t tables, size_t per_sub, int W, int max_block = kBlock) {
+inline int block_threads(size_t tables, size_t per_sub, int W) {
   static int optin = 0;
   if (optin == 0) {
     int dev = 0, v = 0;
@@ -23,9 +23,27 @@ inline int block_threads(size_t tables, size_t per_sub, int W, int max_block = k
     if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess || v <= 0) v = 48 * 1024;
     optin = v;
   }
-  for (int b = max_block; b >= 32; b /= 2)
+  for (int b = kBlock; b >= 32; b /= 2)
     if (tables + (size_t)(b / W) * per_sub <= (size_t)optin) return b;
   return 0;
+}
+
+// CTA size (threads, a multiple of 32 up to max_block) with the most threads on an SM by shared memory,
+// among those with more than `least`; the smallest of equals.  The register limit is the caller's to check.
+inline int widest_block(size_t tables, size_t per_sub, int W, int max_block, int least) {
+  constexpr size_t kPerSm = 228 * 1024, kReserved = 1024;  // shared memory of an SM, and what each CTA costs beside its own
+  int best = kBlock, most = least;
+  for (int b = 64; b <= max_block; b += 32) {
+    const size_t cta = tables + (size_t)(b / W) * per_sub;
+    if (cta + kReserved > kPerSm) break;
+    int n = (int)(kPerSm / (cta + kReserved)) * b;
+    if (n > 512) n = 512;
+    if (n > most) {
+      most = n;
+      best = b;
+    }
+  }
+  return best;
 }
 
 template <typename R, typename RL, int N, int KIND, int V, int S, int WK>
@@ -34,36 +52,53 @@ int launch_track_w(const TrackParams& p, cudaStream_t s, int n_sm) {
   auto kern = dev::track_kernel<R, RL, N, W, KIND, V, S, WK>;
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const int slots = (dev::kFlatAlways<N> || p.flat_eval) ? p.scr_slots : 0;
-  const size_t tables = dev::tables_bytes(N, p.n_hx_terms, p.n_ht_terms, !std::is_same<R, RL>::value);
+  const size_t tables = dev::tables_bytes(N, staged_words(WK, p.n_hx_terms, p.n_hx_rows), p.n_ht_terms, !std::is_same<R, RL>::value);
   const size_t per_sub = dev::sub_bytes(N, Mc, W, slots, 2 * (int)sizeof(RL), 2 * (int)sizeof(R));
-  const int block = block_threads(tables, per_sub, W, GHC_BLOCK(N, R, RL, V));
-  if (block == 0) return -24;
-  const int subs = block / W;
-  const size_t smem = tables + subs * per_sub;
   // Host calls in the launch path delay small launches, so per instantiation and device the
   // shared-memory attribute is only ever raised (to the largest size asked for, so a concurrent
   // launch never sees it below its own size) and the occupancy of the last size is kept.
   constexpr int kDevs = 16;
-  static std::atomic<long long> attr_max[kDevs], occ_key[kDevs];
-  static std::atomic<int> occ_val[kDevs];
+  static std::atomic<long long> attr_max[kDevs], occ_key[kDevs][2];
+  static std::atomic<int> occ_val[kDevs][2];
   int dev_id = 0;
   cudaError_t e = cudaGetDevice(&dev_id);
   if (e != cudaSuccess) return -20;
   const int d = dev_id & (kDevs - 1);
-  long long have = attr_max[d].load();
-  while (have < (long long)smem) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return -20;
-    if (attr_max[d].compare_exchange_weak(have, (long long)smem)) break;
+  // CTAs per SM of `block` threads each; slot: which of the two launch shapes keeps the answer
+  auto occupancy = [&](int block, int slot) -> int {
+    const size_t smem = tables + (size_t)(block / W) * per_sub;
+    long long have = attr_max[d].load();
+    while (have < (long long)smem) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -20;
+      if (attr_max[d].compare_exchange_weak(have, (long long)smem)) break;
+    }
+    const long long okey = (long long)smem * 512 + block + 1;
+    int occ = occ_key[d][slot].load() == okey ? occ_val[d][slot].load() : 0;
+    if (occ < 1) {
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, block, smem) != cudaSuccess || occ < 1) return -21;
+      occ_val[d][slot].store(occ);
+      occ_key[d][slot].store(okey);
+    }
+    return occ;
+  };
+  int block = block_threads(tables, per_sub, W);
+  if (block == 0) return -24;
+  int occ = occupancy(block, 0);
+  if (occ < 0) return occ;
+  if (dev::track_block<N, R, RL, V>() > kBlock && p.n_items > (long long)occ * n_sm * (block / W)) {
+    // more paths than one wave of the usual CTAs: the CTA size that keeps the most paths on an SM
+    const int wide = widest_block(tables, per_sub, W, dev::track_block<N, R, RL, V>(), occ * block);
+    if (wide != block) {
+      const int o = occupancy(wide, 1);
+      if (o < 0) return o;
+      if (o * wide > occ * block) {
+        block = wide;
+        occ = o;
+      }
+    }
   }
-  const long long okey = (long long)smem * 256 + block + 1;
-  int occ = occ_key[d].load() == okey ? occ_val[d].load() : 0;
-  if (occ < 1) {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, block, smem);
-    if (e != cudaSuccess || occ < 1) return -21;
-    occ_val[d].store(occ);
-    occ_key[d].store(okey);
-  }
+  const int subs = block / W;
+  const size_t smem = tables + (size_t)subs * per_sub;
   // persistent grid: fill the GPU once, but never launch more sub-warps than items; a launch
   // with fewer paths than one warp per scheduler of every SM gives each path its own warp
   TrackParams q = p;
@@ -117,7 +152,8 @@ int launch_polish_s(const PolishParams& p, cudaStream_t s) {
   auto kern = dev::polish_kernel<N, W, KIND, S>;
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const int slots = (dev::kFlatAlways<N> || p.flat_eval) ? p.scr_slots : 0;
-  const size_t tables = dev::tables_bytes(N, p.n_hx_terms, p.n_ht_terms, false);
+  const int walk = (dev::kFlatAlways<N> && p.flat_eval == 0) ? 1 : p.flat_eval;
+  const size_t tables = dev::tables_bytes(N, staged_words(walk, p.n_hx_terms, p.n_hx_rows), p.n_ht_terms, false);
   const size_t per_sub = dev::sub_bytes(N, Mc, W, slots, 16, 16);
   const int block = block_threads(tables, per_sub, W);
   if (block == 0) return -24;
