@@ -31,7 +31,7 @@ namespace dev {
 constexpr unsigned kFull = 0xffffffffu;
 
 template <typename R>
-struct cx {
+struct alignas(2 * sizeof(R)) cx {
   R re, im;
 };
 
@@ -202,48 +202,91 @@ __device__ __forceinline__ cx<R> acc_term(cx<R> acc, cx<R> p, uint2 w, const uns
   }
 }
 
+// complex entry of a table of doubles: one 16-byte load where the table is aligned to that (WIDE)
+template <typename R, bool WIDE>
+__device__ __forceinline__ cx<R> ldg_cx(const double* a) {
+  if constexpr (WIDE) {
+    const double2 v = __ldg(reinterpret_cast<const double2*>(a));
+    return mk((R)v.x, (R)v.y);
+  } else {
+    return mk((R)__ldg(a), (R)__ldg(a + 1));
+  }
+}
+// polynomial with complex coefficients a[0..n] at t (Horner)
+template <typename R, bool WIDE, int NN>
+__device__ __forceinline__ cx<R> poly_at(const double* a, int n, R t) {
+  if constexpr (NN >= 0) {  // all loads at once
+    cx<R> v[NN + 1];
+#pragma unroll
+    for (int j = 0; j <= NN; ++j) v[j] = ldg_cx<R, WIDE>(a + 2 * j);
+#pragma unroll
+    for (int j = NN - 1; j >= 0; --j) v[NN] = mk(f_fma(v[NN].re, t, v[j].re), f_fma(v[NN].im, t, v[j].im));
+    return v[NN];
+  } else {
+    cx<R> v = ldg_cx<R, WIDE>(a + 2 * n);
+    for (int j = n - 1; j >= 0; --j) {
+      const cx<R> w = ldg_cx<R, WIDE>(a + 2 * j);
+      v = mk(f_fma(v.re, t, w.re), f_fma(v.im, t, w.im));
+    }
+    return v;
+  }
+}
 // c_k(t), c'_k(t) for k = l, l+W, ... (reference eval_parameter_homotopy), computed in R and
-// stored in RO; with HI the R values of c_k(t) are also kept in hi (the residual's copy)
+// stored in RO; with HI the R values of c_k(t) are also kept in hi (the residual's copy).
+// KK: the polynomials' degree K, or 0 for any.
+template <typename R, typename RO, int W, bool HI, bool WIDE, int KK>
+__device__ __forceinline__ void coef_loop_p2c(const double* __restrict__ hx, const double* __restrict__ ht, int M,
+                                              int K, R t, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l) {
+  const int n = KK > 0 ? KK : K;
+  for (int k = l; k <= M; k += W) {
+    const cx<R> v = poly_at<R, WIDE, (KK > 0 ? KK : -1)>(hx + 2 * (size_t)k * (n + 1), n, t);
+    c[k] = c_cast<RO>(v);
+    if (HI) hi[k] = v;
+    cp[k] = n >= 1 ? c_cast<RO>(poly_at<R, WIDE, KK - 1>(ht + 2 * (size_t)k * n, n - 1, t)) : mk(RO(0), RO(0));
+  }
+}
+// The lanes of a path read its tables entry by entry at a stride of K (+ 1) complex values, so every
+// load touches most lines of the table: half as many loads (whole complex values) are half as many
+// passes over them.  With the shorter path record: P3P one instance FP64 123 -> 105 us, 20,000 hypotheses
+// 2.11 -> 1.88 ms, 5-point 12.3 -> 10.9, gen-3v-4pt 90.5 -> 84.8.
 template <typename R, typename RO, int W, bool HI>
 __device__ __forceinline__ void coef_eval_p2c(const double* __restrict__ hx, const double* __restrict__ ht, int M,
                                               int K, R t, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l) {
-  for (int k = l; k <= M; k += W) {
-    const double* a = hx + 2 * (size_t)k * (K + 1);
-    cx<R> v = mk((R)__ldg(a + 2 * K), (R)__ldg(a + 2 * K + 1));
-    for (int j = K - 1; j >= 0; --j) v = mk(f_fma(v.re, t, (R)__ldg(a + 2 * j)), f_fma(v.im, t, (R)__ldg(a + 2 * j + 1)));
-    c[k] = c_cast<RO>(v);
+  const bool wide = ((reinterpret_cast<uintptr_t>(hx) | reinterpret_cast<uintptr_t>(ht)) & 15) == 0;
+  if (wide && K == 1) coef_loop_p2c<R, RO, W, HI, true, 1>(hx, ht, M, K, t, c, cp, hi, l);
+  else if (wide && K == 2) coef_loop_p2c<R, RO, W, HI, true, 2>(hx, ht, M, K, t, c, cp, hi, l);
+  else coef_loop_p2c<R, RO, W, HI, false, 0>(hx, ht, M, K, t, c, cp, hi, l);
+}
+
+// p(t) = p1 t + p0 (1-t) and, on a new path (fresh), the parameter differences (reference
+// compute_param_homotopy), computed in R and stored in RO; with HI the R values of p(t) are also kept in hi
+template <typename R, typename RO, int W, bool HI, bool WIDE>
+__device__ __forceinline__ void coef_loop_ph(const double* __restrict__ ps, const double* __restrict__ pt,
+                                             const double* __restrict__ pd, int P, R t, bool fresh, cx<RO>* ph,
+                                             cx<RO>* dp, cx<R>* hi, int l) {
+  const R u = f_sub(R(1), t);
+  for (int k = l; k < P; k += W) {
+    const cx<R> g = ldg_cx<R, WIDE>(pt + 2 * k), s = ldg_cx<R, WIDE>(ps + 2 * k);
+    const cx<R> v = mk(f_fma(g.re, t, f_mul(s.re, u)), f_fma(g.im, t, f_mul(s.im, u)));
+    ph[k] = c_cast<RO>(v);
     if (HI) hi[k] = v;
-    if (K >= 1) {
-      const double* b = ht + 2 * (size_t)k * K;
-      cx<R> u = mk((R)__ldg(b + 2 * (K - 1)), (R)__ldg(b + 2 * (K - 1) + 1));
-      for (int j = K - 2; j >= 0; --j) u = mk(f_fma(u.re, t, (R)__ldg(b + 2 * j)), f_fma(u.im, t, (R)__ldg(b + 2 * j + 1)));
-      cp[k] = c_cast<RO>(u);
-    } else {
-      cp[k] = mk(RO(0), RO(0));
+  }
+  if (fresh) {
+    for (int k = l; k <= P; k += W) dp[k] = mk((RO)__ldg(pd + 2 * k), (RO)__ldg(pd + 2 * k + 1));
+    if (l == 0) {
+      ph[P] = mk(RO(1), RO(0));
+      if (HI) hi[P] = mk(R(1), R(0));
     }
   }
 }
-
-// p(t) = p1 t + p0 (1-t) and the parameter differences (reference compute_param_homotopy), computed
-// in R and stored in RO; with HI the R values of p(t) are also kept in hi
 template <typename R, typename RO, int W, bool HI>
 __device__ __forceinline__ void coef_eval_ph(const double* __restrict__ ps, const double* __restrict__ pt,
-                                             const double* __restrict__ pd, int P, R t, cx<RO>* ph, cx<RO>* dp,
-                                             cx<R>* hi, int l) {
-  const R u = f_sub(R(1), t);
-  for (int k = l; k < P; k += W) {
-    const R gr = (R)__ldg(pt + 2 * k), gi = (R)__ldg(pt + 2 * k + 1);
-    const R sr = (R)__ldg(ps + 2 * k), si = (R)__ldg(ps + 2 * k + 1);
-    const cx<R> v = mk(f_fma(gr, t, f_mul(sr, u)), f_fma(gi, t, f_mul(si, u)));
-    ph[k] = c_cast<RO>(v);
-    if (HI) hi[k] = v;
-    dp[k] = mk((RO)__ldg(pd + 2 * k), (RO)__ldg(pd + 2 * k + 1));
-  }
-  if (l == 0) {
-    ph[P] = mk(RO(1), RO(0));
-    if (HI) hi[P] = mk(R(1), R(0));
-    dp[P] = mk((RO)__ldg(pd + 2 * P), (RO)__ldg(pd + 2 * P + 1));
-  }
+                                             const double* __restrict__ pd, int P, R t, bool fresh, cx<RO>* ph,
+                                             cx<RO>* dp, cx<R>* hi, int l) {
+  if (((reinterpret_cast<uintptr_t>(ps) | reinterpret_cast<uintptr_t>(pt)) & 15) == 0)
+    coef_loop_ph<R, RO, W, HI, true>(ps, pt, pd, P, t, fresh, ph, dp, hi, l);
+  else
+    coef_loop_ph<R, RO, W, HI, false>(ps, pt, pd, P, t, fresh, ph, dp, hi, l);
 }
 
 // term value p (coefficient, or product of two homotopy parameters, times the integer scale)
@@ -752,11 +795,12 @@ __device__ __forceinline__ cx<R> lu_solve(cx<R> (&A)[N], cx<R> b, int l, cx<R>* 
   return lu_solve<R, N, W>(A, b, l, sx, sol, rg);
 }
 
-// xor-butterfly sum over the first NP lanes of the sub-warp (order = oracle tree_sum)
+// xor-butterfly sum over the NP = W lanes of the sub-warp (order = oracle tree_sum); the same bits in
+// every lane, for a + b = b + a
 template <typename R, int N, int W>
 __device__ __forceinline__ R tree_sum(R v) {
   constexpr int NP = (N <= 1) ? 1 : (N <= 2) ? 2 : (N <= 4) ? 4 : (N <= 8) ? 8 : (N <= 16) ? 16 : 32;
-  static_assert(NP <= W, "sub-warp narrower than the reduction tree");
+  static_assert(NP == W, "every lane of the sub-warp is a leaf of the reduction tree");
 #pragma unroll
   for (int off = NP / 2; off > 0; off >>= 1) v = f_add(v, shfl_xor(v, off, W));
   return v;
@@ -851,13 +895,13 @@ __device__ __forceinline__ void write_one(const SubMem& sm, int l) {
 }
 
 template <typename R, typename RL, int W, int KIND>
-__device__ __forceinline__ void coef_eval(const TrackParams& p, const SubMem& sm, long long hyp, R t, int l) {
+__device__ __forceinline__ void coef_eval(const TrackParams& p, const SubMem& sm, long long hyp, R t, bool fresh, int l) {
   constexpr bool HI = !std::is_same<R, RL>::value;
   if (KIND == KIND_P2C) {
     coef_eval_p2c<R, RL, W, HI>(p.coef_hx + 2 * hyp * p.stride_hx, p.coef_ht + 2 * hyp * p.stride_ht, p.M, p.K, t,
                                 view<RL>(sm.coefA), view<RL>(sm.coefB), view<R>(sm.coefH), l);
   } else {
-    coef_eval_ph<R, RL, W, HI>(p.p_start, p.p_tgt + 2 * hyp * p.stride_p, p.p_diff + 2 * hyp * p.stride_p, p.P, t,
+    coef_eval_ph<R, RL, W, HI>(p.p_start, p.p_tgt + 2 * hyp * p.stride_p, p.p_diff + 2 * hyp * p.stride_p, p.P, t, fresh,
                                view<RL>(sm.coefA), view<RL>(sm.coefB), view<R>(sm.coefH), l);
   }
 }
@@ -1062,8 +1106,11 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
   const long long n_sw = n_cta * slots_per_cta;
   const bool primary = !p.spread || lane < W;
   const int leader = lane - l;
-  const bool handover = p.t_handover > 0.0 || p.fail_limit > 0;
-  const R t_hand = (R)p.t_handover;
+  // handover rules (first phase of the mixed mode): only the mixed tracker's launch sets them
+  constexpr bool kMixed = !std::is_same<R, RL>::value;
+  const bool handover = kMixed && (p.t_handover > 0.0 || p.fail_limit > 0);
+  const bool by_time = kMixed && p.t_handover > 0.0;
+  const R t_hand = kMixed ? (R)p.t_handover : R(0);
 
   // per-path state (replicated across the sub-warp's lanes)
   long long item = p.spread ? cta * slots_per_cta + (threadIdx.x >> 5) : cta * subs_per_cta + g;
@@ -1079,7 +1126,6 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
   R coef_t = R(-1);  // the t at which this sub-warp's coefficient buffers hold c_k(t) (-1: none)
   bool end_zone = false, success = false, inf = false, finished = false;
   // mixed tracker only: a solve of this step was ill-conditioned, or the step fell below the floor: stop
-  constexpr bool kMixed = !std::is_same<R, RL>::value;
   bool step_ill = false, ill_stop = false;
   bool step_sing = false, last_sing = false;  // a solve of this step / the last completed step had a zero pivot
   int nsucc = 0, step = 0, ncorr = 0, phase = 0, cit = 0, nfail = 0;
@@ -1096,7 +1142,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
       if (dt > edge) dt = edge;
     }
     dt_pre = dt;  // the step without the handover clamp: the next phase resumes with it
-    if (p.t_handover > 0.0 && dt > f_sub(t_hand, t0)) dt = f_sub(t_hand, t0);
+    if (by_time && dt > f_sub(t_hand, t0)) dt = f_sub(t_hand, t0);
     t_step = t0;
     half = f_mul(R(0.5), dt);
     phase = 0;
@@ -1107,7 +1153,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
   // the path stops before its next step (kernel_HC_Solver_P3P.cu:247-249, plus the handover rules)
   auto at_end = [&]() -> bool {
     return !(t0 < R(1) && f_sub(R(1), t0) > R(1e-7)) || step > p.max_steps ||
-           (p.t_handover > 0.0 && f_sub(t_hand, t0) <= R(1e-6)) || (p.fail_limit > 0 && nfail >= p.fail_limit) ||
+           (by_time && f_sub(t_hand, t0) <= R(1e-6)) || (kMixed && p.fail_limit > 0 && nfail >= p.fail_limit) ||
            (kMixed && ill_stop);
   };
   auto init_path = [&](long long it) {
@@ -1143,45 +1189,47 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
 
   // The path's scalar state (the same in every lane of the sub-warp) and this lane's track
   // component wait in shared memory while the sub-warp evaluates and solves, so that no
-  // register holds them across the LU (register relief).  Volatile: stored and reloaded,
-  // never forwarded.
-  volatile R* rec_r = reinterpret_cast<volatile R*>(sm.rec);
-  volatile long long* rec_l = reinterpret_cast<volatile long long*>(sm.rec + 6 * sizeof(R));
-  volatile int* rec_i = reinterpret_cast<volatile int*>(sm.rec + 6 * sizeof(R) + 2 * sizeof(long long));
+  // register holds them across the LU (register relief; the synchronisations between keep the
+  // compiler from forwarding them).  In as few and as wide accesses as they fit in.
+  cx<R>* const rec_r = view<R>(sm.rec);                                             // 3 complex
+  int4* const rec_i = reinterpret_cast<int4*>(sm.rec + 48);                         // 1
+  uint2* const rec_u = reinterpret_cast<uint2*>(sm.rec + 64);                       // 2
   auto stash = [&]() {
-    rec_r[0] = t0;
-    rec_r[1] = dt;
-    rec_r[2] = t_step;
-    rec_r[3] = half;
-    rec_r[4] = dt_pre;
-    rec_r[5] = coef_t;
-    rec_l[0] = item;
-    rec_l[1] = hyp;
-    rec_i[0] = step;
-    rec_i[1] = ncorr;
-    rec_i[2] = phase;
-    rec_i[3] = cit;
-    rec_i[4] = nfail;
-    rec_i[5] = nsucc;
-    rec_i[6] = (alive ? 1 : 0) | (finished ? 2 : 0) | (end_zone ? 4 : 0) | (success ? 8 : 0) | (inf ? 16 : 0) |
-               (step_ill ? 32 : 0) | (ill_stop ? 64 : 0) | (step_sing ? 128 : 0) | (last_sing ? 256 : 0);
+    rec_r[0] = mk(t0, dt);
+    rec_r[1] = mk(t_step, coef_t);
+    rec_i[0] = make_int4(step, ncorr, cit, nsucc);
+    rec_u[0] = make_uint2((unsigned)item, (unsigned)hyp);
+    const unsigned f = (alive ? 1 : 0) | (finished ? 2 : 0) | (end_zone ? 4 : 0) | (success ? 8 : 0) | (inf ? 16 : 0) |
+                       (step_ill ? 32 : 0) | (ill_stop ? 64 : 0) | (step_sing ? 128 : 0) | (last_sing ? 256 : 0) |
+                       (unsigned)phase << 9;
+    if (kMixed) {
+      rec_r[2] = mk(dt_pre, R(0));
+      rec_u[1] = make_uint2(f, (unsigned)nfail);
+    } else {
+      rec_u[1].x = f;
+    }
   };
   auto unstash = [&]() {
-    t0 = rec_r[0];
-    dt = rec_r[1];
-    t_step = rec_r[2];
-    half = rec_r[3];
-    dt_pre = rec_r[4];
-    coef_t = rec_r[5];
-    item = rec_l[0];
-    hyp = rec_l[1];
-    step = rec_i[0];
-    ncorr = rec_i[1];
-    phase = rec_i[2];
-    cit = rec_i[3];
-    nfail = rec_i[4];
-    nsucc = rec_i[5];
-    const int f = rec_i[6];
+    const cx<R> a = rec_r[0], b = rec_r[1];
+    t0 = a.re;
+    dt = a.im;
+    t_step = b.re;
+    coef_t = b.im;
+    half = f_mul(R(0.5), dt);  // as the step's prologue set it (dt does not change within a step)
+    const int4 n = rec_i[0];
+    step = n.x;
+    ncorr = n.y;
+    cit = n.z;
+    nsucc = n.w;
+    const uint2 u = rec_u[0];
+    item = u.x;
+    hyp = u.y;
+    const unsigned f = rec_u[1].x;
+    if (kMixed) {
+      dt_pre = rec_r[2].re;
+      nfail = (int)rec_u[1].y;
+    }
+    phase = (int)(f >> 9);
     alive = f & 1;
     finished = (f >> 1) & 1;
     end_zone = (f >> 2) & 1;
@@ -1191,8 +1239,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
     ill_stop = (f >> 6) & 1;
     step_sing = (f >> 7) & 1;
     last_sing = (f >> 8) & 1;
-    const volatile cx<R>* xv = reinterpret_cast<const volatile cx<R>*>(sm.xst);
-    x = (l < N) ? mk(xv[l].re, xv[l].im) : mk(R(0), R(0));
+    x = (l < N) ? view<R>(sm.xst)[l] : mk(R(0), R(0));
   };
 
   while (__any_sync(kFull, alive)) {
@@ -1203,7 +1250,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
     // (RK stages 2 and 3 share t + dt/2, and after an accepted step the next step starts at the t
     // of the last stage, whose coefficients are still in the buffers: evaluate only on a new t)
     if (rk && t0 != coef_t) {
-      coef_eval<R, RL, W, KIND>(p, sm, hyp, t0, l);
+      coef_eval<R, RL, W, KIND>(p, sm, hyp, t0, coef_t == R(-1), l);
       coef_t = t0;
     }
     // ---------------- one evaluate-and-solve per sub-warp (predictor: -H_t, corrector: H)
@@ -1221,8 +1268,8 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
       const cx<R> xn = c_sub(x, v);
       const R ns = tree_sum<R, N, W>((corr && l < N) ? c_abs2(v) : R(0));
       const R nc = tree_sum<R, N, W>((corr && l < N) ? c_abs2(xn) : R(0));
-      ns0 = __shfl_sync(kFull, ns, leader);
-      nc0 = __shfl_sync(kFull, nc, leader);
+      ns0 = ns;
+      nc0 = nc;
     }
     // ---------------- per-sub-warp state update (no synchronisation below until the fetch)
     bool end_step = false;
@@ -1283,13 +1330,14 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
       if (kMixed && (step_ill || (p.dt_floor > 0.0 && (double)dt < p.dt_floor))) ill_stop = true;
       last_sing = step_sing;
       if (!done) done = at_end();
-      if (done && !inf && p.t_handover > 0.0 && f_sub(t_hand, t0) <= R(1e-6) && step <= p.max_steps &&
+      if (done && !inf && by_time && f_sub(t_hand, t0) <= R(1e-6) && step <= p.max_steps &&
           dt < dt_pre)
         dt = dt_pre;
       if (!done) prologue();
     }
 
     // ---------------- finished paths: write out and take the next path
+    if (!__any_sync(kFull, done)) continue;
     // (a non-finite track anywhere in the sub-warp; every lane takes part in the vote)
     const unsigned bad = __ballot_sync(kFull, l < N && !(isfinite(x.re) && isfinite(x.im)));
     const bool nonfinite = ((W == 32 ? bad : bad >> leader) & (W == 32 ? kFull : ((1u << (W & 31)) - 1u))) != 0u;
@@ -1314,7 +1362,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
         // a path handed over at the boundary resumes at exactly t_handover, not at its float t
         // (a float t just short of the boundary would put the next step just short of the end
         // zone, where the edge clamp shrinks dt to the gap)
-        const bool boundary = p.t_handover > 0.0 && !inf && f_sub(t_hand, t0) <= R(1e-6);
+        const bool boundary = by_time && !inf && f_sub(t_hand, t0) <= R(1e-6);
         if (p.t_end) p.t_end[item] = boundary ? p.t_handover : (double)t0;
         if (p.dt_end) p.dt_end[item] = (double)dt;
       }
@@ -1374,7 +1422,7 @@ __global__ void __launch_bounds__(128) polish_kernel(const PolishParams p) {
                                                 nullptr, l);
       } else {
         coef_eval_ph<double, double, W, false>(p.p_start, p.p_tgt + 2 * hyp * p.stride_p,
-                                               p.p_diff + 2 * hyp * p.stride_p, p.P, 1.0, view<double>(sm.coefA),
+                                               p.p_diff + 2 * hyp * p.stride_p, p.P, 1.0, true, view<double>(sm.coefA),
                                                view<double>(sm.coefB), nullptr, l);
       }
     }
