@@ -236,14 +236,16 @@ __device__ __forceinline__ cx<R> poly_at(const double* a, int n, R t) {
 // KK: the polynomials' degree K, or 0 for any.
 template <typename R, typename RO, int W, bool HI, bool WIDE, int KK>
 __device__ __forceinline__ void coef_loop_p2c(const double* __restrict__ hx, const double* __restrict__ ht, int M,
-                                              int K, R t, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l) {
+                                              int K, R t, bool fresh, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l) {
   const int n = KK > 0 ? KK : K;
   for (int k = l; k <= M; k += W) {
     const cx<R> v = poly_at<R, WIDE, (KK > 0 ? KK : -1)>(hx + 2 * (size_t)k * (n + 1), n, t);
     c[k] = c_cast<RO>(v);
     if (HI) hi[k] = v;
-    cp[k] = n >= 1 ? c_cast<RO>(poly_at<R, WIDE, KK - 1>(ht + 2 * (size_t)k * n, n - 1, t)) : mk(RO(0), RO(0));
+    if (KK != 1) cp[k] = n >= 1 ? c_cast<RO>(poly_at<R, WIDE, KK - 1>(ht + 2 * (size_t)k * n, n - 1, t)) : mk(RO(0), RO(0));
   }
+  if (KK == 1 && fresh)  // constant in t: written for the path's first evaluation
+    for (int k = l; k <= M; k += W) cp[k] = c_cast<RO>(ldg_cx<R, WIDE>(ht + 2 * (size_t)k));
 }
 // The lanes of a path read its tables entry by entry at a stride of K (+ 1) complex values, so every
 // load touches most lines of the table: half as many loads (whole complex values) are half as many
@@ -251,11 +253,11 @@ __device__ __forceinline__ void coef_loop_p2c(const double* __restrict__ hx, con
 // 2.11 -> 1.88 ms, 5-point 12.3 -> 10.9, gen-3v-4pt 90.5 -> 84.8.
 template <typename R, typename RO, int W, bool HI>
 __device__ __forceinline__ void coef_eval_p2c(const double* __restrict__ hx, const double* __restrict__ ht, int M,
-                                              int K, R t, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l) {
+                                              int K, R t, bool fresh, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l) {
   const bool wide = ((reinterpret_cast<uintptr_t>(hx) | reinterpret_cast<uintptr_t>(ht)) & 15) == 0;
-  if (wide && K == 1) coef_loop_p2c<R, RO, W, HI, true, 1>(hx, ht, M, K, t, c, cp, hi, l);
-  else if (wide && K == 2) coef_loop_p2c<R, RO, W, HI, true, 2>(hx, ht, M, K, t, c, cp, hi, l);
-  else coef_loop_p2c<R, RO, W, HI, false, 0>(hx, ht, M, K, t, c, cp, hi, l);
+  if (wide && K == 1) coef_loop_p2c<R, RO, W, HI, true, 1>(hx, ht, M, K, t, fresh, c, cp, hi, l);
+  else if (wide && K == 2) coef_loop_p2c<R, RO, W, HI, true, 2>(hx, ht, M, K, t, fresh, c, cp, hi, l);
+  else coef_loop_p2c<R, RO, W, HI, false, 0>(hx, ht, M, K, t, fresh, c, cp, hi, l);
 }
 
 // p(t) = p1 t + p0 (1-t) and, on a new path (fresh), the parameter differences (reference
@@ -464,9 +466,10 @@ template <int N>
 constexpr int kLuForm = N <= GHC_LU_SERIAL_MAX_N ? LU_SERIAL : LU_GROUPED;
 // Columns per group: a smaller group wastes fewer updates beyond the shrinking row (a group's columns
 // all run at its first one's width), a larger one is less code and less shared memory.  B200, ms:
-// N = 6 (five-point FP64) 13.61 at 2, 13.66 at 3, 13.82 at 1, 13.88 at 6; N = 12 (gen-3v-4pt FP64)
-// 93.7 at 4, 95.3 at 3, 102.6 at 2 and 108.5 at 6; N = 30 FP64 115.4 at 10, 124.9 at 6, 131 at 15.
-__host__ __device__ constexpr int lu_group(int N) { return N <= 6 ? 2 : N <= 16 ? 4 : N <= 18 ? 6 : 10; }
+// N = 6 (five-point FP64) 10.64 at 1, 10.90 at 2, 11.21 at 6; N = 12 gen-3v-4pt FP64 83.5 at 3, 83.3 at
+// 2, 83.8 at 4, 85.4 at 6, mixed 34.6, 35.1, 34.8, 36.9; N = 30 FP64 109.0 at 5, 112.0 at 6, 110.3 at
+// 10, 114.1 at 3, FP32 67.0 at 5 and 6, 69.3 at 3, 71.8 at 10.
+__host__ __device__ constexpr int lu_group(int N) { return N <= 6 ? 1 : N <= 16 ? 3 : N <= 18 ? 6 : 5; }
 // stored pivot rows of a group that starts with rows of w entries: even stride (with the right-hand
 // side at entry w), so that the back substitution's diagonal reads fall into different banks
 __host__ __device__ constexpr int lu_row_stride(int w) { return (w + 2) & ~1; }
@@ -669,23 +672,22 @@ __device__ __forceinline__ cx<R> lu_solve_grouped(cx<R> (&A)[N], cx<R> b, int l,
       } else if (pos == i) {
         pos = bp;
       }
-      const cx<R> f = c_mul(A[0], rc);
-      if (__any_sync(kFull, pm == R(0))) {  // rare: a path of the warp skips the column
-        const bool skip = pm == R(0);
-        static_for<0, w - 1>([&](auto jc) {
-          constexpr int j = decltype(jc)::value;
-          const cx<R> u = c_fnma(f, px[j + 1], A[j + 1]);
-          A[j] = skip ? A[j + 1] : u;
-        });
-        const cx<R> u = c_fnma(f, px[w], b);
-        b = skip ? b : u;
-      } else {
-        static_for<0, w - 1>([&](auto jc) {
-          constexpr int j = decltype(jc)::value;
-          if (has(std::integral_constant<int, j + 1>{})) A[j] = c_fnma(f, px[j + 1], A[j + 1]);
-        });
-        b = c_fnma(f, px[w], b);
+      cx<R> f = c_mul(A[0], rc);
+      if (__any_sync(kFull, pm == R(0))) {
+        // Rare: a path of the warp skips the column.  Its update takes zero times a row of zeros from
+        // every entry, which leaves them (a zero may lose its sign); the stored row is not needed, for
+        // the NaN reciprocal makes its component NaN whatever the row holds.
+        if (pm == R(0)) {
+          f = mk(R(0), R(0));
+          for (int k = l; k <= w; k += W) px[k] = f;
+        }
+        __syncwarp(kFull);
       }
+      static_for<0, w - 1>([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        if (has(std::integral_constant<int, j + 1>{})) A[j] = c_fnma(f, px[j + 1], A[j + 1]);
+      });
+      b = c_fnma(f, px[w], b);
     }
   });
   __syncwarp(kFull);  // the pivot rows and reciprocals are stored
@@ -822,7 +824,7 @@ struct SubMem {
   unsigned nz;           // this lane's row: bit i set when H_x entry (row, i) has terms
   int walk;              // H_x walk: 0 entry-wise, 1 row-wise, 2 balanced
 };
-constexpr int kRecBytes = 128;
+constexpr int kRecBytes = 80;
 
 // bit i set when row r of H_x has terms in column i (0 for lanes beyond the rows)
 template <int N>
@@ -898,7 +900,7 @@ template <typename R, typename RL, int W, int KIND>
 __device__ __forceinline__ void coef_eval(const TrackParams& p, const SubMem& sm, long long hyp, R t, bool fresh, int l) {
   constexpr bool HI = !std::is_same<R, RL>::value;
   if (KIND == KIND_P2C) {
-    coef_eval_p2c<R, RL, W, HI>(p.coef_hx + 2 * hyp * p.stride_hx, p.coef_ht + 2 * hyp * p.stride_ht, p.M, p.K, t,
+    coef_eval_p2c<R, RL, W, HI>(p.coef_hx + 2 * hyp * p.stride_hx, p.coef_ht + 2 * hyp * p.stride_ht, p.M, p.K, t, fresh,
                                 view<RL>(sm.coefA), view<RL>(sm.coefB), view<R>(sm.coefH), l);
   } else {
     coef_eval_ph<R, RL, W, HI>(p.p_start, p.p_tgt + 2 * hyp * p.stride_p, p.p_diff + 2 * hyp * p.stride_p, p.P, t, fresh,
@@ -917,7 +919,9 @@ __host__ __device__ inline size_t tables_bytes(int N, int n_hx, int n_ht, bool m
 // [slots W] (flat) in the same place as the solve scratch [lu_scratch_len(N)]; the coefficient buffers
 // [2 Mc] and, mixed, the state-precision coefficients [Mc].  What the problem's tables do not size
 // comes first, so its offsets are constants of the kernel.  An odd multiple of 16 bytes: equal places
-// of two sub-warps never fall into the same banks.
+// of two sub-warps never fall into the same banks; with 4 lanes three or five eighths of a bank row
+// apart, so that the windows of four complex values which neighbouring sub-warps read overlap least
+// (P3P FP64, 20,000 hypotheses: 1.80 ms at 48 bytes beyond a multiple of 128, 1.90 at 112, 2.03 at 64).
 struct SubOffsets {
   size_t coefA, coefB, xs, sx, sol, state, scr, coefH, xsH, bytes;
 };
@@ -928,7 +932,7 @@ __host__ __device__ inline SubOffsets sub_offsets(int N, int Mc, int W, int slot
   o.xs = off;
   off += (size_t)e * (N + 1);
   o.sol = off;
-  off = align16(off + (size_t)e * N);
+  off = align16(off + (N <= GHC_LU_SERIAL_MAX_N ? 0 : (size_t)e * N));
   o.state = off;
   off += (size_t)es * 2 * W;
   o.xsH = 0;
@@ -949,6 +953,8 @@ __host__ __device__ inline SubOffsets sub_offsets(int N, int Mc, int W, int slot
     off += (size_t)es * Mc;
   }
   o.bytes = align16(off) | 16;
+  if (W == 4)
+    while (o.bytes % 128 != 48 && o.bytes % 128 != 80) o.bytes += 16;
   return o;
 }
 __host__ __device__ inline size_t sub_bytes(int N, int Mc, int W, int slots, int e, int es) {
@@ -1418,7 +1424,7 @@ __global__ void __launch_bounds__(128) polish_kernel(const PolishParams p) {
     if (conv) {
       if (KIND == KIND_P2C) {
         coef_eval_p2c<double, double, W, false>(p.coef_hx + 2 * hyp * p.stride_hx, p.coef_ht + 2 * hyp * p.stride_ht,
-                                                p.M, p.K, 1.0, view<double>(sm.coefA), view<double>(sm.coefB),
+                                                p.M, p.K, 1.0, true, view<double>(sm.coefA), view<double>(sm.coefB),
                                                 nullptr, l);
       } else {
         coef_eval_ph<double, double, W, false>(p.p_start, p.p_tgt + 2 * hyp * p.stride_p,
