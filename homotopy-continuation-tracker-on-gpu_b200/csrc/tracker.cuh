@@ -231,64 +231,64 @@ __device__ __forceinline__ cx<R> poly_at(const double* a, int n, R t) {
     return v;
   }
 }
-// c_k(t), c'_k(t) for k = l, l+W, ... (reference eval_parameter_homotopy), computed in R and
+// c_k(t), c'_k(t) for k = l, l + step, ... (reference eval_parameter_homotopy), computed in R and
 // stored in RO; with HI the R values of c_k(t) are also kept in hi (the residual's copy).
 // KK: the polynomials' degree K, or 0 for any.
-template <typename R, typename RO, int W, bool HI, bool WIDE, int KK>
+template <typename R, typename RO, bool HI, bool WIDE, int KK>
 __device__ __forceinline__ void coef_loop_p2c(const double* __restrict__ hx, const double* __restrict__ ht, int M,
-                                              int K, R t, bool fresh, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l) {
+                                              int K, R t, bool fresh, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l, int step) {
   const int n = KK > 0 ? KK : K;
-  for (int k = l; k <= M; k += W) {
+  for (int k = l; k <= M; k += step) {
     const cx<R> v = poly_at<R, WIDE, (KK > 0 ? KK : -1)>(hx + 2 * (size_t)k * (n + 1), n, t);
     c[k] = c_cast<RO>(v);
     if (HI) hi[k] = v;
     if (KK != 1) cp[k] = n >= 1 ? c_cast<RO>(poly_at<R, WIDE, KK - 1>(ht + 2 * (size_t)k * n, n - 1, t)) : mk(RO(0), RO(0));
   }
   if (KK == 1 && fresh)  // constant in t: written for the path's first evaluation
-    for (int k = l; k <= M; k += W) cp[k] = c_cast<RO>(ldg_cx<R, WIDE>(ht + 2 * (size_t)k));
+    for (int k = l; k <= M; k += step) cp[k] = c_cast<RO>(ldg_cx<R, WIDE>(ht + 2 * (size_t)k));
 }
 // The lanes of a path read its tables entry by entry at a stride of K (+ 1) complex values, so every
 // load touches most lines of the table: half as many loads (whole complex values) are half as many
 // passes over them.  With the shorter path record: P3P one instance FP64 123 -> 105 us, 20,000 hypotheses
 // 2.11 -> 1.88 ms, 5-point 12.3 -> 10.9, gen-3v-4pt 90.5 -> 84.8.
-template <typename R, typename RO, int W, bool HI>
+template <typename R, typename RO, bool HI>
 __device__ __forceinline__ void coef_eval_p2c(const double* __restrict__ hx, const double* __restrict__ ht, int M,
-                                              int K, R t, bool fresh, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l) {
+                                              int K, R t, bool fresh, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l, int step) {
   const bool wide = ((reinterpret_cast<uintptr_t>(hx) | reinterpret_cast<uintptr_t>(ht)) & 15) == 0;
-  if (wide && K == 1) coef_loop_p2c<R, RO, W, HI, true, 1>(hx, ht, M, K, t, fresh, c, cp, hi, l);
-  else if (wide && K == 2) coef_loop_p2c<R, RO, W, HI, true, 2>(hx, ht, M, K, t, fresh, c, cp, hi, l);
-  else coef_loop_p2c<R, RO, W, HI, false, 0>(hx, ht, M, K, t, fresh, c, cp, hi, l);
+  if (wide && K == 1) coef_loop_p2c<R, RO, HI, true, 1>(hx, ht, M, K, t, fresh, c, cp, hi, l, step);
+  else if (wide && K == 2) coef_loop_p2c<R, RO, HI, true, 2>(hx, ht, M, K, t, fresh, c, cp, hi, l, step);
+  else coef_loop_p2c<R, RO, HI, false, 0>(hx, ht, M, K, t, fresh, c, cp, hi, l, step);
 }
 
 // p(t) = p1 t + p0 (1-t) and, on a new path (fresh), the parameter differences (reference
 // compute_param_homotopy), computed in R and stored in RO; with HI the R values of p(t) are also kept in hi
-template <typename R, typename RO, int W, bool HI, bool WIDE>
+template <typename R, typename RO, bool HI, bool WIDE>
 __device__ __forceinline__ void coef_loop_ph(const double* __restrict__ ps, const double* __restrict__ pt,
                                              const double* __restrict__ pd, int P, R t, bool fresh, cx<RO>* ph,
-                                             cx<RO>* dp, cx<R>* hi, int l) {
+                                             cx<RO>* dp, cx<R>* hi, int l, int step) {
   const R u = f_sub(R(1), t);
-  for (int k = l; k < P; k += W) {
+  for (int k = l; k < P; k += step) {
     const cx<R> g = ldg_cx<R, WIDE>(pt + 2 * k), s = ldg_cx<R, WIDE>(ps + 2 * k);
     const cx<R> v = mk(f_fma(g.re, t, f_mul(s.re, u)), f_fma(g.im, t, f_mul(s.im, u)));
     ph[k] = c_cast<RO>(v);
     if (HI) hi[k] = v;
   }
   if (fresh) {
-    for (int k = l; k <= P; k += W) dp[k] = mk((RO)__ldg(pd + 2 * k), (RO)__ldg(pd + 2 * k + 1));
+    for (int k = l; k <= P; k += step) dp[k] = mk((RO)__ldg(pd + 2 * k), (RO)__ldg(pd + 2 * k + 1));
     if (l == 0) {
       ph[P] = mk(RO(1), RO(0));
       if (HI) hi[P] = mk(R(1), R(0));
     }
   }
 }
-template <typename R, typename RO, int W, bool HI>
+template <typename R, typename RO, bool HI>
 __device__ __forceinline__ void coef_eval_ph(const double* __restrict__ ps, const double* __restrict__ pt,
                                              const double* __restrict__ pd, int P, R t, bool fresh, cx<RO>* ph,
-                                             cx<RO>* dp, cx<R>* hi, int l) {
+                                             cx<RO>* dp, cx<R>* hi, int l, int step) {
   if (((reinterpret_cast<uintptr_t>(ps) | reinterpret_cast<uintptr_t>(pt)) & 15) == 0)
-    coef_loop_ph<R, RO, W, HI, true>(ps, pt, pd, P, t, fresh, ph, dp, hi, l);
+    coef_loop_ph<R, RO, HI, true>(ps, pt, pd, P, t, fresh, ph, dp, hi, l, step);
   else
-    coef_loop_ph<R, RO, W, HI, false>(ps, pt, pd, P, t, fresh, ph, dp, hi, l);
+    coef_loop_ph<R, RO, HI, false>(ps, pt, pd, P, t, fresh, ph, dp, hi, l, step);
 }
 
 // term value p (coefficient, or product of two homotopy parameters, times the integer scale)
@@ -353,7 +353,7 @@ __device__ __forceinline__ cx<R> eval_rhs(const uint2* terms, const uint16_t* of
 
 template <typename R, int N, int W, int KIND, int NVX>
 __device__ __forceinline__ void eval_row(const Tables& tb, const unsigned char* ca, const unsigned char* xs, int r,
-                                         bool live, cx<R> (&A)[N], int walk, unsigned char* scr, unsigned nz) {
+                                         bool live, cx<R> (&A)[N], int walk, uint2 seg, unsigned char* scr, unsigned nz) {
   // the row's k-th non-zero entry waits in slot k (W complex values each) until the row is read back
   auto read_back = [&]() {
     const cx<R>* sp = view<R>(scr) + r;
@@ -377,10 +377,10 @@ __device__ __forceinline__ void eval_row(const Tables& tb, const unsigned char* 
       A[i] = acc;
     }
   } else if (balanced) {
-    // this lane's share of the entries (every lane of the sub-warp takes part); each finished
-    // sum goes into the slot of its row, read back after the sub-warp synchronises
-    const uint2* wp = tb.hx_terms + r;  // (the staged section is the balanced one)
-    const int len = tb.hx_off[N * N + 2 + r];
+    // this lane's share of the entries (every lane takes part); each finished sum goes into the slot of
+    // its row, read back after the sub-warp synchronises
+    const int len = (int)(seg.x >> 16);
+    const uint2* wp = tb.hx_terms + r + (seg.x & 0xffffu) * W;  // (the staged section is the balanced one)
     cx<R> acc = mk(R(0), R(0));
 #pragma unroll 4
     for (int q = 0; q < len; ++q) {
@@ -395,9 +395,9 @@ __device__ __forceinline__ void eval_row(const Tables& tb, const unsigned char* 
     read_back();
   } else {
     if (live) {
-      const uint2* wp = tb.hx_terms + r;
-      const int len = tb.hx_off[r * N + N] - tb.hx_off[r * N];
-      cx<R>* sp = view<R>(scr) + r;
+      const int len = (int)(seg.x >> 16);
+      const uint2* wp = tb.hx_terms + r + (seg.x & 0xffffu) * N;
+      cx<R>* sp = view<R>(scr) + r + seg.y * W;
       cx<R> acc = mk(R(0), R(0));
 #pragma unroll 4
       for (int q = 0; q < len; ++q) {
@@ -410,8 +410,7 @@ __device__ __forceinline__ void eval_row(const Tables& tb, const unsigned char* 
         }
       }
     }
-    // row-wise: this lane's own slots (each walk reads back inside its own branch: a read-back
-    // shared by the walks after the branches cost hundreds of bytes of register spills)
+    __syncwarp(kFull);  // (a spread path's other sub-warps wrote slots of this row too)
     read_back();
   }
 }
@@ -817,6 +816,7 @@ struct SubMem {
   unsigned char* sol;    // pivot reciprocals [N]
   unsigned char* state;  // per lane: RK base point x0 [W], RK accumulator [W] (state precision)
   unsigned char* scr;    // H_x row scratch [slots][W] of the flat walks, in the solve scratch's place
+  unsigned char* seg;    // per lane: the terms of its H_x walk, first | number << 16, and the first one's slot [W]
   unsigned char* rec;    // the path's scalar state while the sub-warp evaluates and solves [kRecBytes]
   unsigned char* coefH;  // mixed: c_k(t) or p(t) in state precision, for the residual H [Mc] (else null)
   unsigned char* xsH;    // mixed: the track in state precision [N+1] (else null)
@@ -836,6 +836,29 @@ __device__ __forceinline__ unsigned row_mask(const uint16_t* hx_off, int r) {
   return m;
 }
 
+// This lane's part of the H_x walk: all of its list (row l, or, balanced, the l-th share), or, for one of
+// `parts` sub-warps that evaluate one path together, the part-th piece of it, cut between entries.
+template <int N, int W, int NVX>
+__device__ __forceinline__ uint2 walk_range(const Tables& tb, int walk, int l, int part, int parts) {
+  const bool balanced = balanced_walk_built(N) && walk == 2 && tb.hx_off[N * N + 1] != kNoLanes;
+  const int len = balanced ? tb.hx_off[N * N + 2 + l] : l < N ? tb.hx_off[l * N + N] - tb.hx_off[l * N] : 0;
+  const int stride = balanced ? W : N;
+  int first = len, end = len, slot = 0, slots = 0;
+  for (int q = 0; q <= len; ++q) {  // q: a place where an entry begins (or the list ends)
+    if (q > 0 && !word_last<NVX>(tb.hx_terms[(q - 1) * stride + l])) continue;
+    if (q > 0) ++slots;
+    if (first == len && q * parts >= len * part) {
+      first = q;
+      slot = slots;
+    }
+    if (q * parts >= len * (part + 1)) {
+      end = q;
+      break;
+    }
+  }
+  return make_uint2((unsigned)first | (unsigned)(end - first) << 16, (unsigned)slot);
+}
+
 // Row l of H_x and the right-hand side (which = 1: -H_t, which = 0: H), term walk of table shape S
 // (EvalShape), in the linear-algebra precision RL.  With a state precision R above RL (mixed), the
 // corrector's H is evaluated in R from the R copies of the coefficients and the track, then rounded
@@ -843,7 +866,8 @@ __device__ __forceinline__ unsigned row_mask(const uint16_t* hx_off, int r) {
 template <typename R, typename RL, int N, int W, int KIND, int S>
 __device__ __forceinline__ void eval_any(const Tables& tb, const SubMem& sm, int l, cx<RL> (&A)[N], cx<RL>& b,
                                          int which) {
-  eval_row<RL, N, W, KIND, shape_nvx(S)>(tb, sm.coefA, sm.xs, l, l < N, A, sm.walk, sm.scr, sm.nz);
+  eval_row<RL, N, W, KIND, shape_nvx(S)>(tb, sm.coefA, sm.xs, l, l < N, A, sm.walk, reinterpret_cast<const uint2*>(sm.seg)[l],
+                                         sm.scr, sm.nz);
   if constexpr (std::is_same<R, RL>::value) {
     b = eval_rhs<RL, N, KIND, shape_nvt(S)>(tb.ht_terms, tb.ht_off, sm.coefA, sm.coefB, sm.xs, l, l < N, which);
   } else {
@@ -897,14 +921,14 @@ __device__ __forceinline__ void write_one(const SubMem& sm, int l) {
 }
 
 template <typename R, typename RL, int W, int KIND>
-__device__ __forceinline__ void coef_eval(const TrackParams& p, const SubMem& sm, long long hyp, R t, bool fresh, int l) {
+__device__ __forceinline__ void coef_eval(const TrackParams& p, const SubMem& sm, long long hyp, R t, bool fresh, int l, int step) {
   constexpr bool HI = !std::is_same<R, RL>::value;
   if (KIND == KIND_P2C) {
-    coef_eval_p2c<R, RL, W, HI>(p.coef_hx + 2 * hyp * p.stride_hx, p.coef_ht + 2 * hyp * p.stride_ht, p.M, p.K, t, fresh,
-                                view<RL>(sm.coefA), view<RL>(sm.coefB), view<R>(sm.coefH), l);
+    coef_eval_p2c<R, RL, HI>(p.coef_hx + 2 * hyp * p.stride_hx, p.coef_ht + 2 * hyp * p.stride_ht, p.M, p.K, t, fresh,
+                                view<RL>(sm.coefA), view<RL>(sm.coefB), view<R>(sm.coefH), l, step);
   } else {
-    coef_eval_ph<R, RL, W, HI>(p.p_start, p.p_tgt + 2 * hyp * p.stride_p, p.p_diff + 2 * hyp * p.stride_p, p.P, t, fresh,
-                               view<RL>(sm.coefA), view<RL>(sm.coefB), view<R>(sm.coefH), l);
+    coef_eval_ph<R, RL, HI>(p.p_start, p.p_tgt + 2 * hyp * p.stride_p, p.p_diff + 2 * hyp * p.stride_p, p.P, t, fresh,
+                               view<RL>(sm.coefA), view<RL>(sm.coefB), view<R>(sm.coefH), l, step);
   }
 }
 
@@ -913,7 +937,7 @@ __host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~(size_t
 __host__ __device__ inline size_t tables_bytes(int N, int n_hx, int n_ht, bool mixed) {
   return align16(8 * ((size_t)n_hx + (mixed ? 2 : 1) * (size_t)n_ht) + 2 * (size_t)(hx_off_len(N) + N + 1));
 }
-// Per sub-warp: the path record [kRecBytes], then, in complex values of e bytes (linear-algebra
+// Per sub-warp: the path record [kRecBytes], the lanes' walk ranges [W], then, in complex values of e bytes (linear-algebra
 // precision): track [N+1], pivot reciprocals [N]; the lane state [2 W] and, when es != e (mixed), the
 // state-precision track [N+1] in complex values of es bytes (state precision); the row scratch
 // [slots W] (flat) in the same place as the solve scratch [lu_scratch_len(N)]; the coefficient buffers
@@ -923,12 +947,14 @@ __host__ __device__ inline size_t tables_bytes(int N, int n_hx, int n_ht, bool m
 // apart, so that the windows of four complex values which neighbouring sub-warps read overlap least
 // (P3P FP64, 20,000 hypotheses: 1.80 ms at 48 bytes beyond a multiple of 128, 1.90 at 112, 2.03 at 64).
 struct SubOffsets {
-  size_t coefA, coefB, xs, sx, sol, state, scr, coefH, xsH, bytes;
+  size_t seg, coefA, coefB, xs, sx, sol, state, scr, coefH, xsH, bytes;
 };
 __host__ __device__ inline SubOffsets sub_offsets(int N, int Mc, int W, int slots, int e, int es) {
   const bool mixed = es != e;
   SubOffsets o;
   size_t off = kRecBytes;
+  o.seg = off;
+  off += 8 * (size_t)W;
   o.xs = off;
   off += (size_t)e * (N + 1);
   o.sol = off;
@@ -965,6 +991,7 @@ __device__ __forceinline__ SubMem sub_layout(unsigned char* base, int N, int Mc,
   const SubOffsets o = sub_offsets(N, Mc, W, flat ? slots : 0, (int)sizeof(cx<RL>), (int)sizeof(cx<R>));
   SubMem sm;
   sm.rec = base;
+  sm.seg = base + o.seg;
   sm.coefA = base + o.coefA;
   sm.coefB = base + o.coefB;
   sm.xs = base + o.xs;
@@ -1098,6 +1125,22 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
   sm.nz = row_mask<N>(tb.hx_off, l);
   sm.walk = walk;
   write_one<R, RL, N>(sm, l);
+  // Spread, all sub-warps of the warp have the same path: they share one copy of the coefficients and
+  // of the row scratch, and each evaluates a part of both, which shortens the chain of a lone path
+  // (B200, one instance: P3P FP64 107 -> 92 us, 5-point FP32 2.19 -> 1.57 ms, gen-3v-4pt FP32
+  // 1.09 -> 1.00).  What a sub-warp updates in place, and its solve, stay its own.
+  reinterpret_cast<uint2*>(sm.seg)[l] =
+      walk_range<N, W, shape_nvx(S)>(tb, walk, l, p.spread ? lane / W : 0, p.spread ? 32 / W : 1);
+  if (p.spread) {
+    const SubMem first = sub_layout<R, RL>(
+        smem + tables_bytes(N, n_hx, p.n_ht_terms, !std::is_same<R, RL>::value) +
+            (size_t)(g - lane / W) * sub_bytes(N, Mc, W, flat ? p.scr_slots : 0, (int)sizeof(cx<RL>), (int)sizeof(cx<R>)),
+        N, Mc, W, p.scr_slots, flat);
+    sm.coefA = first.coefA;
+    sm.coefB = first.coefB;
+    sm.coefH = first.coefH;
+    sm.scr = first.scr;
+  }
   // this lane's RK base point x0 and accumulator sols live in shared memory (register relief)
   cx<R>& x0 = view<R>(sm.state)[l];
   cx<R>& sols = view<R>(sm.state)[W + l];
@@ -1198,8 +1241,8 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
   // register holds them across the LU (register relief; the synchronisations between keep the
   // compiler from forwarding them).  In as few and as wide accesses as they fit in.
   cx<R>* const rec_r = view<R>(sm.rec);                                             // 3 complex
-  int4* const rec_i = reinterpret_cast<int4*>(sm.rec + 48);                         // 1
-  uint2* const rec_u = reinterpret_cast<uint2*>(sm.rec + 64);                       // 2
+  int4* const rec_i = reinterpret_cast<int4*>(sm.rec + kRecBytes - 32);
+  uint2* const rec_u = reinterpret_cast<uint2*>(sm.rec + kRecBytes - 16);
   auto stash = [&]() {
     rec_r[0] = mk(t0, dt);
     rec_r[1] = mk(t_step, coef_t);
@@ -1256,7 +1299,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
     // (RK stages 2 and 3 share t + dt/2, and after an accepted step the next step starts at the t
     // of the last stage, whose coefficients are still in the buffers: evaluate only on a new t)
     if (rk && t0 != coef_t) {
-      coef_eval<R, RL, W, KIND>(p, sm, hyp, t0, coef_t == R(-1), l);
+      coef_eval<R, RL, W, KIND>(p, sm, hyp, t0, coef_t == R(-1), p.spread ? lane : l, p.spread ? 32 : W);
       coef_t = t0;
     }
     // ---------------- one evaluate-and-solve per sub-warp (predictor: -H_t, corrector: H)
@@ -1411,6 +1454,7 @@ __global__ void __launch_bounds__(128) polish_kernel(const PolishParams p) {
   sm.nz = row_mask<N>(tb.hx_off, l);
   sm.walk = walk;
   write_one<double, double, N>(sm, l);
+  reinterpret_cast<uint2*>(sm.seg)[l] = walk_range<N, W, shape_nvx(S)>(tb, walk, l, 0, 1);
   const int subs_per_cta = blockDim.x / W;
   const int leader = lane - l;
   for (long long item0 = (long long)blockIdx.x * subs_per_cta; item0 < p.n_items;
@@ -1423,13 +1467,13 @@ __global__ void __launch_bounds__(128) polish_kernel(const PolishParams p) {
     cx<double> x = (valid && l < N) ? mk(ep[2 * l], ep[2 * l + 1]) : mk(0.0, 0.0);
     if (conv) {
       if (KIND == KIND_P2C) {
-        coef_eval_p2c<double, double, W, false>(p.coef_hx + 2 * hyp * p.stride_hx, p.coef_ht + 2 * hyp * p.stride_ht,
+        coef_eval_p2c<double, double, false>(p.coef_hx + 2 * hyp * p.stride_hx, p.coef_ht + 2 * hyp * p.stride_ht,
                                                 p.M, p.K, 1.0, true, view<double>(sm.coefA), view<double>(sm.coefB),
-                                                nullptr, l);
+                                                nullptr, l, W);
       } else {
-        coef_eval_ph<double, double, W, false>(p.p_start, p.p_tgt + 2 * hyp * p.stride_p,
+        coef_eval_ph<double, double, false>(p.p_start, p.p_tgt + 2 * hyp * p.stride_p,
                                                p.p_diff + 2 * hyp * p.stride_p, p.P, 1.0, true, view<double>(sm.coefA),
-                                               view<double>(sm.coefB), nullptr, l);
+                                               view<double>(sm.coefB), nullptr, l, W);
       }
     }
     __syncwarp(kFull);
