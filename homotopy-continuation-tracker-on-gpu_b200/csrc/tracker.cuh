@@ -1074,7 +1074,7 @@ __device__ __forceinline__ Tables stage_tables(unsigned char* smem, const uint64
 //
 // Each sub-warp runs its path as a small state machine (phase 0..3 = RK stage,
 // 4 = Newton iteration).  One trip of the warp loop performs exactly one
-// evaluate-and-solve for every sub-warp, whatever its phase, so the unrolled
+// evaluate-and-solve for every sub-warp, whatever its phase, so the
 // LU exists once in the code and sub-warps of one warp never wait on each
 // other's corrector iterations.
 //
