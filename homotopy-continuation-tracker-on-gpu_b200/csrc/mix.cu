@@ -26,6 +26,7 @@
 #include "abi_internal.h"
 #include "ghc_internal.h"
 #include "problem.h"
+#include "smem_limit.h"
 #include "tracker.cuh"
 
 namespace ghc {
@@ -150,8 +151,7 @@ extern "C" int ghc_track_mix(const ghc_problem* const* pbs, const ghc_track_args
   int any = 0;
   for (int k = 0; k < kMixSlots; ++k) any |= mp.used[k];
   if (!any) return GHC_OK;
-  if (cudaFuncSetAttribute(mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return cuda_fail("ghc_track_mix: shared memory");
+  if (!allow_smem<mix_kernel>()) return cuda_fail("ghc_track_mix: shared memory");
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mix_kernel, kMixBlock, smem) != cudaSuccess || occ < 1)
     return cuda_fail("ghc_track_mix: occupancy");

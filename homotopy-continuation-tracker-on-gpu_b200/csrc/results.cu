@@ -25,6 +25,7 @@
 #include <cstdint>
 
 #include "ghc_internal.h"
+#include "smem_limit.h"
 
 namespace ghc {
 namespace {
@@ -220,14 +221,11 @@ int launch_t(int N, int paths, long long n_hyp, const double* z, const uint8_t* 
              double imag_tol, double dup_tol, int* counts, uint8_t* cls, cudaStream_t s) {
   constexpr int kGroups = T == 32 ? kWarps : 1;
   const size_t smem = kGroups * group_bytes(paths, T, STAGED);
-  auto kern = results_kernel<T, STAGED>;
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return -20;
+  if (smem > 48 * 1024 && !allow_smem<results_kernel<T, STAGED>>()) return -20;
   long long grid = (n_hyp + kGroups - 1) / kGroups;
   if (grid > 148LL * 32) grid = 148LL * 32;
-  kern<<<(unsigned)grid, T == 32 ? 32 * kWarps : T, smem, s>>>(N, paths, n_hyp, z, conv, inf, imag_tol, dup_tol,
-                                                               counts, cls);
+  results_kernel<T, STAGED><<<(unsigned)grid, T == 32 ? 32 * kWarps : T, smem, s>>>(
+      N, paths, n_hyp, z, conv, inf, imag_tol, dup_tol, counts, cls);
   return cudaGetLastError() == cudaSuccess ? 0 : -23;
 }
 

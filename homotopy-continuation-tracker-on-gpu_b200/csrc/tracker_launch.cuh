@@ -5,6 +5,7 @@
 #include <atomic>
 
 #include "ghc_internal.h"
+#include "smem_limit.h"
 #include "tracker.cuh"
 
 namespace ghc {
@@ -56,23 +57,18 @@ int launch_track_w(const TrackParams& p, cudaStream_t s, int n_sm) {
   const size_t tables = dev::tables_bytes(N, staged_words(WK, p.n_hx_terms, p.n_hx_rows), p.n_ht_terms, !std::is_same<R, RL>::value);
   const size_t per_sub = dev::sub_bytes(N, Mc, W, slots, 2 * (int)sizeof(RL), 2 * (int)sizeof(R));
   // Host calls in the launch path delay small launches, so per instantiation and device the
-  // shared-memory attribute is only ever raised (to the largest size asked for, so a concurrent
-  // launch never sees it below its own size) and the occupancy of the last size is kept.
+  // occupancy of the last size is kept.
   constexpr int kDevs = 16;
-  static std::atomic<long long> attr_max[kDevs], occ_key[kDevs][2];
+  static std::atomic<long long> occ_key[kDevs][2];
   static std::atomic<int> occ_val[kDevs][2];
   int dev_id = 0;
   cudaError_t e = cudaGetDevice(&dev_id);
   if (e != cudaSuccess) return -20;
   const int d = dev_id & (kDevs - 1);
+  if (!allow_smem<dev::track_kernel<R, RL, N, W, KIND, V, S, WK>>()) return -20;
   // CTAs per SM of `block` threads each; slot: which of the two launch shapes keeps the answer
   auto occupancy = [&](int block, int slot) -> int {
     const size_t smem = tables + (size_t)(block / W) * per_sub;
-    long long have = attr_max[d].load();
-    while (have < (long long)smem) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -20;
-      if (attr_max[d].compare_exchange_weak(have, (long long)smem)) break;
-    }
     const long long okey = (long long)smem * 512 + block + 1;
     int occ = occ_key[d][slot].load() == okey ? occ_val[d][slot].load() : 0;
     if (occ < 1) {
@@ -160,7 +156,7 @@ int launch_polish_s(const PolishParams& p, cudaStream_t s) {
   if (block == 0) return -24;
   const int subs = block / W;
   const size_t smem = tables + subs * per_sub;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -20;
+  if (!allow_smem<dev::polish_kernel<N, W, KIND, S>>()) return -20;
   long long grid = (p.n_items + subs - 1) / subs;
   if (grid > 65535LL * 16) grid = 65535LL * 16;
   if (grid < 1) grid = 1;
