@@ -119,6 +119,17 @@ PolishParams polish_params(const TrackParams& t, double* endpoints, const uint8_
   return q;
 }
 
+// A launch hands its paths out by a 32-bit counter (the caller's d_counter) and keeps a path's number
+// in 32 bits while it is tracked; one path beyond 2^32 the counter would wrap and the launch never end.
+int check_items(const Problem& pb, int64_t n_hyp, int32_t paths) {
+  const int64_t per_hyp = paths > 0 ? paths : pb.paths;
+  if (n_hyp > (int64_t{1} << 32) / per_hyp) {
+    set_error("more than 2^32 paths in one launch");
+    return GHC_ERR_RANGE;
+  }
+  return GHC_OK;
+}
+
 int track_params(const Problem& pb, const ghc_track_args* a, TrackParams& p) {
   p = base_params(pb);
   apply_tuning(pb, a->precision, p);
@@ -496,8 +507,8 @@ int ghc_track(const ghc_problem* h, const ghc_track_args* a, void* stream) {
     return GHC_ERR_ARG;
   }
   Problem& pb = const_cast<Problem&>(h->pb);
-  int rc = ensure_device(pb);
-  if (rc) return rc;
+  int rc = check_items(pb, a->n_hyp, a->paths);
+  if (rc || (rc = ensure_device(pb))) return rc;
   TrackParams p;
   if ((rc = track_params(pb, a, p))) return rc;
   return run_track(p, a, stream);
@@ -738,8 +749,8 @@ int ghc_solve_host(const ghc_problem* h, int32_t precision, int64_t n_hyp, const
   }
   Problem& pb = const_cast<Problem&>(h->pb);
   if (!h_targets) n_hyp = 1;
-  int rc = ensure_device(pb);
-  if (rc) return rc;
+  int rc = check_items(pb, n_hyp, 0);
+  if (rc || (rc = ensure_device(pb))) return rc;
   const bool fp32 = precision == GHC_PREC_FP32;
   const long long n = n_hyp * (long long)pb.paths;
   const int N = pb.N, P1 = pb.P + 1;

@@ -17,6 +17,8 @@ int cuda_fail(const char* what);    // GHC_ERR_CUDA with the last CUDA error as 
 int track_code(int rc);             // launch_track / launch_polish codes -> GHC_* with a message
 TrackParams base_params(const Problem& pb);
 PolishParams polish_params(const TrackParams& t, double* endpoints, const uint8_t* conv, double* resid, int iters);
+// Refuses (GHC_ERR_RANGE) a launch of more paths than the 32-bit work counter numbers.
+int check_items(const Problem& pb, int64_t n_hyp, int32_t paths);
 // The launch parameters of a ghc_track call: the problem's sizes, tuning and device tables
 // (pb.dev), the caller's buffers and step control, a->d_counter as the work-stealing counter.
 int track_params(const Problem& pb, const ghc_track_args* a, TrackParams& p);

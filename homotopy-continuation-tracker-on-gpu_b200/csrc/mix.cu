@@ -134,8 +134,8 @@ extern "C" int ghc_track_mix(const ghc_problem* const* pbs, const ghc_track_args
                 "(2,3) term shapes; " + pb.name + (k < 0 ? " is none of them" : " repeats a bucket"));
       return GHC_ERR_RANGE;
     }
-    int rc = ensure_device(pb);
-    if (rc) return rc;
+    int rc = check_items(pb, a->n_hyp, a->paths);
+    if (rc || (rc = ensure_device(pb))) return rc;
     TrackParams& p = mp.b[k];
     if ((rc = track_params(pb, a, p))) return rc;
     p.spread = 0;

@@ -92,6 +92,8 @@ extern "C" int ghc_track_noalloc(const ghc_problem* h, const ghc_track_args* a, 
     return GHC_ERR_ARG;
   }
   const Problem& pb = h->pb;
+  int rc = check_items(pb, a->n_hyp, a->paths);
+  if (rc) return rc;
   // scratch layout: [counter | hx terms | hx offsets | ht terms | ht offsets]
   const size_t o_hx = 256;
   const size_t o_hxo = o_hx + up16(pb.hx_terms.size() * sizeof(uint64_t));
@@ -107,8 +109,7 @@ extern "C" int ghc_track_noalloc(const ghc_problem* h, const ghc_track_args* a, 
   ghc_track_args args = *a;
   args.d_counter = nullptr;  // the array's own counter
   TrackParams p;
-  int rc = track_params(pb, &args, p);
-  if (rc) return rc;
+  if ((rc = track_params(pb, &args, p))) return rc;
   int dev = 0;
   void* base = nullptr;
   if ((rc = scratch_address(&dev, &base))) return rc;

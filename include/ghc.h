@@ -114,7 +114,7 @@ int ghc_p2c_device(const ghc_problem* pb, int64_t n_hyp, const double* d_start, 
  * (GPU-HC/magmaHC/gpu-kernels/magmaHC-kernels.hpp; e.g.
  * kernel_HC_Solver_P3P.cu:267-377 and kernel_HC_Solver_trifocal_2op1p_30x30.cu:313-486)
  * for n_hyp hypotheses x paths in one launch.  Work item i tracks start path
- * i % paths of hypothesis i / paths.
+ * i % paths of hypothesis i / paths.  At most 2^32 paths per launch (more: GHC_ERR_RANGE).
  * ------------------------------------------------------------------------- */
 typedef struct {
   int64_t n_hyp;
