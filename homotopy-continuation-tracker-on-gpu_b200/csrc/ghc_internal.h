@@ -88,7 +88,7 @@ inline int row_nonzeros_max(const uint16_t* hx_off, int N) {
 inline int row_words(const uint16_t* hx_off, int N, int n_hx) {
   return hx_off[N * N + 1] == kNoLanes ? n_hx : hx_off[N * N + 1];
 }
-// words that a CTA stages for a walk: only the section that the walk reads
+// H_x words that a CTA stages for a walk: only the section that the walk reads
 GHC_HD inline int staged_words(int walk, int n_hx, int n_rows) { return walk == 2 && n_rows < n_hx ? n_hx - n_rows : n_rows; }
 
 inline int flat_eval_pays(const uint16_t* hx_off, int N) {
@@ -130,8 +130,10 @@ inline int flat_eval_pays(const uint16_t* hx_off, int N) {
 // Term shape of a problem: (variable slots per H_x term, per H_t term).  Every term of a
 // table has parts - 1 - (coefficient slots) variable slots (compile_tables keeps slot N,
 // the constant 1); the two shapes of the shipped problems get kernels with straight-line
-// term evaluation, any other shape the general kernel.
-enum EvalShape : int { EVAL_GENERAL = 0, EVAL_1_2 = 1, EVAL_2_3 = 2 };
+// term evaluation, any other shape the general kernel.  EVAL_IN_PLACE is the general walk over
+// term words left in device memory, for launches whose words and path buffers do not fit into one
+// CTA's shared memory together (never a problem's own shape).
+enum EvalShape : int { EVAL_GENERAL = 0, EVAL_1_2 = 1, EVAL_2_3 = 2, EVAL_IN_PLACE = 3 };
 inline int eval_shape_of(int kind, int Px, int Pt) {
   const int c = kind == KIND_PH ? 2 : 1, a = Px - 1 - c, b = Pt - 1 - c;
   return (a == 1 && b == 2) ? EVAL_1_2 : (a == 2 && b == 3) ? EVAL_2_3 : EVAL_GENERAL;

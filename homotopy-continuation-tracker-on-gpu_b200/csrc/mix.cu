@@ -113,6 +113,7 @@ extern "C" int ghc_track_mix(const ghc_problem* const* pbs, const ghc_track_args
   }
   MixParams mp;
   std::memset(&mp, 0, sizeof(mp));
+  const ghc_track_args* own[kMixSlots] = {};
   double weight[kMixSlots] = {0, 0, 0, 0};
   size_t smem = 0;
   cudaStream_t st = (cudaStream_t)stream;
@@ -141,6 +142,7 @@ extern "C" int ghc_track_mix(const ghc_problem* const* pbs, const ghc_track_args
     p.spread = 0;
     mp.used[k] = a->n_hyp > 0 && p.n_items > 0;
     if (!mp.used[k]) continue;
+    own[k] = a;
     if (cudaMemsetAsync(p.counter, 0, sizeof(int), st) != cudaSuccess) return cuda_fail("ghc_track_mix: counter");
     const size_t b = k == 0 ? slot_smem<Slot0>(p) : k == 1 ? slot_smem<Slot1>(p) : k == 2 ? slot_smem<Slot2>(p)
                                                                                     : slot_smem<Slot3>(p);
@@ -151,6 +153,13 @@ extern "C" int ghc_track_mix(const ghc_problem* const* pbs, const ghc_track_args
   int any = 0;
   for (int k = 0; k < kMixSlots; ++k) any |= mp.used[k];
   if (!any) return GHC_OK;
+  if (smem > cta_smem_limit()) {  // a bucket that only its own launch has room for: every bucket its own
+    for (int k = 0; k < kMixSlots; ++k) {
+      const int rc = mp.used[k] ? run_track(mp.b[k], own[k], stream) : GHC_OK;
+      if (rc) return rc;
+    }
+    return GHC_OK;
+  }
   if (!allow_smem<mix_kernel>()) return cuda_fail("ghc_track_mix: shared memory");
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mix_kernel, kMixBlock, smem) != cudaSuccess || occ < 1)

@@ -932,6 +932,16 @@ __device__ __forceinline__ void coef_eval(const TrackParams& p, const SubMem& sm
   }
 }
 
+// term words that a CTA of table shape S stages (EVAL_IN_PLACE: none)
+template <int S>
+__host__ __device__ inline int hx_words(int walk, int n_hx, int n_rows) {
+  return S == EVAL_IN_PLACE ? 0 : staged_words(walk, n_hx, n_rows);
+}
+template <int S>
+__host__ __device__ inline int ht_words(int n_ht) {
+  return S == EVAL_IN_PLACE ? 0 : n_ht;
+}
+
 // byte sizes of the shared-memory layout
 __host__ __device__ inline size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
 __host__ __device__ inline size_t tables_bytes(int N, int n_hx, int n_ht, bool mixed) {
@@ -1042,9 +1052,10 @@ __device__ __forceinline__ Tables stage_tables(unsigned char* smem, const uint64
                                                int n_ht, int walk) {
   constexpr bool mixed = !std::is_same<R, RL>::value;
   constexpr int W = subwarp_width(N), NVX = shape_nvx(S), NVT = shape_nvt(S);
-  uint2* s_hx = reinterpret_cast<uint2*>(smem);
   if (walk == 2 && n_rows < n_hx) g_hx += n_rows;
-  n_hx = staged_words(walk, n_hx, n_rows);
+  n_hx = hx_words<S>(walk, n_hx, n_rows);
+  n_ht = ht_words<S>(n_ht);
+  uint2* s_hx = reinterpret_cast<uint2*>(smem);
   uint2* s_ht = s_hx + n_hx;
   uint2* s_hth = mixed ? s_ht + n_ht : s_ht;
   uint16_t* s_hxo = reinterpret_cast<uint16_t*>(s_hth + n_ht);
@@ -1059,10 +1070,15 @@ __device__ __forceinline__ Tables stage_tables(unsigned char* smem, const uint64
   for (int i = threadIdx.x; i < N + 1; i += blockDim.x) s_hto[i] = __ldg(g_hto + i);
   __syncthreads();
   Tables t;
-  t.hx_terms = s_hx;
+  if constexpr (S == EVAL_IN_PLACE) {
+    t.hx_terms = reinterpret_cast<const uint2*>(g_hx);
+    t.ht_terms = t.ht_terms_hi = reinterpret_cast<const uint2*>(g_ht);
+  } else {
+    t.hx_terms = s_hx;
+    t.ht_terms = s_ht;
+    t.ht_terms_hi = s_hth;
+  }
   t.hx_off = s_hxo;
-  t.ht_terms = s_ht;
-  t.ht_terms_hi = s_hth;
   t.ht_off = s_hto;
   return t;
 }
@@ -1109,7 +1125,7 @@ template <typename R, typename RL, int N, int W, int KIND, int S, int WK>
 __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* smem, long long cta, long long n_cta,
                                            bool visitor) {
   const int walk = WK >= 0 ? WK : ((kFlatAlways<N> && p.flat_eval == 0) ? 1 : p.flat_eval);
-  const int n_hx = staged_words(walk, p.n_hx_terms, p.n_hx_rows);
+  const int n_hx = hx_words<S>(walk, p.n_hx_terms, p.n_hx_rows), n_ht = ht_words<S>(p.n_ht_terms);
   const Tables tb = stage_tables<R, RL, N, KIND, S>(smem, p.hx_terms, p.hx_off, p.ht_terms, p.ht_off, p.n_hx_terms,
                                                     p.n_hx_rows, p.n_ht_terms, walk);
 
@@ -1118,7 +1134,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
   const int g = threadIdx.x / W;
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const bool flat = walk != 0;
-  SubMem sm = sub_layout<R, RL>(smem + tables_bytes(N, n_hx, p.n_ht_terms, !std::is_same<R, RL>::value) +
+  SubMem sm = sub_layout<R, RL>(smem + tables_bytes(N, n_hx, n_ht, !std::is_same<R, RL>::value) +
                                     (size_t)g * sub_bytes(N, Mc, W, flat ? p.scr_slots : 0, (int)sizeof(cx<RL>),
                                                           (int)sizeof(cx<R>)),
                                 N, Mc, W, p.scr_slots, flat);
@@ -1133,7 +1149,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
       walk_range<N, W, shape_nvx(S)>(tb, walk, l, p.spread ? lane / W : 0, p.spread ? 32 / W : 1);
   if (p.spread) {
     const SubMem first = sub_layout<R, RL>(
-        smem + tables_bytes(N, n_hx, p.n_ht_terms, !std::is_same<R, RL>::value) +
+        smem + tables_bytes(N, n_hx, n_ht, !std::is_same<R, RL>::value) +
             (size_t)(g - lane / W) * sub_bytes(N, Mc, W, flat ? p.scr_slots : 0, (int)sizeof(cx<RL>), (int)sizeof(cx<R>)),
         N, Mc, W, p.scr_slots, flat);
     sm.coefA = first.coefA;
@@ -1440,7 +1456,7 @@ template <int N, int W, int KIND, int S>
 __global__ void __launch_bounds__(128) polish_kernel(const PolishParams p) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int walk = (kFlatAlways<N> && p.flat_eval == 0) ? 1 : p.flat_eval;
-  const int n_hx = staged_words(walk, p.n_hx_terms, p.n_hx_rows);
+  const int n_hx = hx_words<S>(walk, p.n_hx_terms, p.n_hx_rows), n_ht = ht_words<S>(p.n_ht_terms);
   const Tables tb = stage_tables<double, double, N, KIND, S>(smem, p.hx_terms, p.hx_off, p.ht_terms, p.ht_off,
                                                              p.n_hx_terms, p.n_hx_rows, p.n_ht_terms, walk);
   const int lane = threadIdx.x & 31;
@@ -1448,7 +1464,7 @@ __global__ void __launch_bounds__(128) polish_kernel(const PolishParams p) {
   const int g = threadIdx.x / W;
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const bool flat = walk != 0;
-  SubMem sm = sub_layout<double, double>(smem + tables_bytes(N, n_hx, p.n_ht_terms, false) +
+  SubMem sm = sub_layout<double, double>(smem + tables_bytes(N, n_hx, n_ht, false) +
                                              (size_t)g * sub_bytes(N, Mc, W, flat ? p.scr_slots : 0, 16, 16),
                                          N, Mc, W, p.scr_slots, flat);
   sm.nz = row_mask<N>(tb.hx_off, l);

@@ -48,13 +48,20 @@ inline int widest_block(size_t tables, size_t per_sub, int W, int max_block, int
   return best;
 }
 
+// A launch whose term words and path buffers do not fit into one CTA even at 32 threads reads the words
+// where they are (EVAL_IN_PLACE; the same sums in the same order).  The words then come through L1, which
+// is slower, so no other launch does; and the walk is the one that needs the least shared memory:
+// entry-wise, where that is built.
+constexpr int in_place_walk(int N) { return N > 16 ? 1 : 0; }
+
 template <typename R, typename RL, int N, int KIND, int V, int S, int WK>
 int launch_track_w(const TrackParams& p, cudaStream_t s, int n_sm) {
   constexpr int W = (N <= 4) ? 4 : (N <= 8) ? 8 : (N <= 16) ? 16 : 32;
   auto kern = dev::track_kernel<R, RL, N, W, KIND, V, S, WK>;
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const int slots = (dev::kFlatAlways<N> || p.flat_eval) ? p.scr_slots : 0;
-  const size_t tables = dev::tables_bytes(N, staged_words(WK, p.n_hx_terms, p.n_hx_rows), p.n_ht_terms, !std::is_same<R, RL>::value);
+  const size_t tables = dev::tables_bytes(N, dev::hx_words<S>(WK, p.n_hx_terms, p.n_hx_rows),
+                                          dev::ht_words<S>(p.n_ht_terms), !std::is_same<R, RL>::value);
   const size_t per_sub = dev::sub_bytes(N, Mc, W, slots, 2 * (int)sizeof(RL), 2 * (int)sizeof(R));
   // Host calls in the launch path delay small launches, so per instantiation and device the
   // occupancy of the last size is kept.
@@ -79,7 +86,14 @@ int launch_track_w(const TrackParams& p, cudaStream_t s, int n_sm) {
     return occ;
   };
   int block = block_threads(tables, per_sub, W);
-  if (block == 0) return -24;
+  if (block == 0) {
+    if constexpr (S != EVAL_IN_PLACE) {
+      TrackParams q = p;
+      q.flat_eval = in_place_walk(N);
+      return launch_track_w<R, RL, N, KIND, V, EVAL_IN_PLACE, in_place_walk(N)>(q, s, n_sm);
+    }
+    return -24;
+  }
   int occ = occupancy(block, 0);
   if (occ < 0) return occ;
   if (dev::track_block<N, R, RL, V>() > kBlock && p.n_items > (long long)occ * n_sm * (block / W)) {
@@ -150,10 +164,18 @@ int launch_polish_s(const PolishParams& p, cudaStream_t s) {
   const int Mc = (KIND == KIND_P2C) ? p.M + 1 : p.P + 1;
   const int slots = (dev::kFlatAlways<N> || p.flat_eval) ? p.scr_slots : 0;
   const int walk = (dev::kFlatAlways<N> && p.flat_eval == 0) ? 1 : p.flat_eval;
-  const size_t tables = dev::tables_bytes(N, staged_words(walk, p.n_hx_terms, p.n_hx_rows), p.n_ht_terms, false);
+  const size_t tables = dev::tables_bytes(N, dev::hx_words<S>(walk, p.n_hx_terms, p.n_hx_rows),
+                                          dev::ht_words<S>(p.n_ht_terms), false);
   const size_t per_sub = dev::sub_bytes(N, Mc, W, slots, 16, 16);
   const int block = block_threads(tables, per_sub, W);
-  if (block == 0) return -24;
+  if (block == 0) {
+    if constexpr (S != EVAL_IN_PLACE) {
+      PolishParams q = p;
+      q.flat_eval = in_place_walk(N);
+      return launch_polish_s<N, KIND, EVAL_IN_PLACE>(q, s);
+    }
+    return -24;
+  }
   const int subs = block / W;
   const size_t smem = tables + subs * per_sub;
   if (!allow_smem<dev::polish_kernel<N, W, KIND, S>>()) return -20;
