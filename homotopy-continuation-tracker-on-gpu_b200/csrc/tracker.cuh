@@ -1254,7 +1254,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
 
   // The path's scalar state (the same in every lane of the sub-warp) and this lane's track
   // component wait in shared memory while the sub-warp evaluates and solves, so that no
-  // register holds them across the LU (register relief; the synchronisations between keep the
+  // register holds them across the LU (register relief; the evaluation's synchronisations keep the
   // compiler from forwarding them).  In as few and as wide accesses as they fit in.
   cx<R>* const rec_r = view<R>(sm.rec);                                             // 3 complex
   int4* const rec_i = reinterpret_cast<int4*>(sm.rec + kRecBytes - 32);
@@ -1320,8 +1320,8 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
     }
     // ---------------- one evaluate-and-solve per sub-warp (predictor: -H_t, corrector: H)
     write_track<R, RL, N>(sm, l, x);
-    stash();
     __syncwarp(kFull);
+    stash();  // (after the synchronisation: a lane may still be reading the last trip's record before it)
     bool ill = false, sing = false;
     const cx<R> v = eval_solve<R, RL, N, W, KIND, S>(tb, sm, l, rk ? 1 : 0, p.cond_limit, ill, sing);
     unstash();
