@@ -100,17 +100,19 @@ inline int flat_eval_pays(const uint16_t* hx_off, int N) {
   if (hx_off[N * N + 1] != kNoLanes) {
     // The balanced walk moves the same shared-memory traffic onto more lanes and scatters the
     // sums: by default only where the rows are uneven.  B200, ms, entry-wise / row-wise / balanced,
-    // by longest row over longest lane.  Up to 8 unknowns it pays from 1.2: 6-line 3-view (1.20,
-    // 16 hypotheses) 237 / 232 / 215, 3-point homography (1.21, 3,000) 6.69 / 5.73 / 5.67, PnP by
-    // quaternions (1.31, 500) 14.8 / 14.4 / 12.8, TDOA (1.33, 600) 19.0 / 18.3 / 17.6, 3-view
-    // triangulation (1.33, 1,500) 4.96 / 4.25 / 4.11; against 6-point rolling shutter (1.20, 1,000)
-    // 3.70 / 3.69 / 3.75.  Above, from 1.4: 4-view triangulation (1.71, 400) 15.9 / 12.2 / 12.0,
+    // by longest row over longest lane.  Up to 8 unknowns it pays above 1.2: 3-point homography
+    // (1.21, 3,000) 6.69 / 5.73 / 5.67, PnP by quaternions (1.31, 500) 14.8 / 14.4 / 12.8, TDOA (1.33,
+    // 600) 19.0 / 18.3 / 17.6, 3-view triangulation (1.33, 1,500) 4.96 / 4.25 / 4.11.  At 1.2 it depends on
+    // how much longer the rows are: 6-line 3-view (40 terms, 66 hypotheses) 712 / 699 / 658, mixed 802 /
+    // 784 / 731, against 6-point rolling shutter (4 terms, 2,000) 7.23 / 7.22 / 7.28, FP32 4.62 / 5.18 /
+    // 5.19, mixed 7.30 / 7.93 / 7.95 (a lone instance 0.50 / 0.42 / 0.44).  Above 8 unknowns, from 1.4: 4-view triangulation (1.71, 400) 15.9 / 12.2 / 12.0,
     // P3P 10x10 (1.64, 2,000) 38.3 / 31.2 / 28.8; gen-3v-4pt (1.33, 128) 29.8 / 21.8 / 22.8, CY
     // (1.22, 32) 33.2 / 25.6 / 26.4, 30x30 (1.28, 16) - / 42.7 / 47.4.
     int lane = 0;
     for (int l = 0; l < subwarp_width(N); ++l)
       if (hx_off[N * N + 2 + l] > lane) lane = hx_off[N * N + 2 + l];
-    if (subwarp_width(N) <= 8 && 10 * longest >= 12 * lane) return 2;
+    const int over = 10 * longest - 12 * lane;
+    if (subwarp_width(N) <= 8 && (over > 0 || (over == 0 && longest - lane >= 16))) return 2;
     if (10 * longest >= 14 * lane) {
       longest = lane;
       walk = 2;

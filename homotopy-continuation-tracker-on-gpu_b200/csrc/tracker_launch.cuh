@@ -141,6 +141,13 @@ int launch_track_s(const TrackParams& p, cudaStream_t s, int n_sm) {
     // one kernel per walk here too: only the chosen walk's code is in the loop body
     if (p.flat_eval == 2 && balanced_walk_built(N)) return launch_track_w<R, RL, N, KIND, V, S, 2>(p, s, n_sm);
     if (p.flat_eval != 0) return launch_track_w<R, RL, N, KIND, V, S, 1>(p, s, n_sm);
+    if (p.n_items <= (long long)n_sm * (kBlock / 32)) {
+      // paths with a warp each: its sub-warps share the rows' walk, which the entry-wise one is not built for
+      // (6-point rolling shutter, one instance, FP64 / FP32 / mixed ms: 0.50 / 0.44 / 0.48 -> 0.42 / 0.37 / 0.42)
+      TrackParams q = p;
+      q.flat_eval = 1;
+      return launch_track_w<R, RL, N, KIND, V, S, 1>(q, s, n_sm);
+    }
     return launch_track_w<R, RL, N, KIND, V, S, 0>(p, s, n_sm);
   }
 }
