@@ -466,9 +466,13 @@ constexpr int kLuForm = N <= GHC_LU_SERIAL_MAX_N ? LU_SERIAL : LU_GROUPED;
 // Columns per group: a smaller group wastes fewer updates beyond the shrinking row (a group's columns
 // all run at its first one's width), a larger one is less code and less shared memory.  B200, ms:
 // N = 6 (five-point FP64) 10.64 at 1, 10.90 at 2, 11.21 at 6; N = 12 gen-3v-4pt FP64 83.5 at 3, 83.3 at
-// 2, 83.8 at 4, 85.4 at 6, mixed 34.6, 35.1, 34.8, 36.9; N = 30 FP64 109.0 at 5, 112.0 at 6, 110.3 at
-// 10, 114.1 at 3, FP32 67.0 at 5 and 6, 69.3 at 3, 71.8 at 10.
-__host__ __device__ constexpr int lu_group(int N) { return N <= 6 ? 1 : N <= 16 ? 3 : N <= 18 ? 6 : 5; }
+// 2, 83.8 at 4, 85.4 at 6, mixed 34.6, 35.1, 34.8, 36.9; N = 18 (6-point rolling shutter, one line, 187
+// hypotheses) FP64 15.9 at 3, 15.7 at 2, 16.5 at 6, 17.1 at 9, FP32 11.2, 11.3, 11.5, 11.6, mixed 14.7, 14.8,
+// 15.1, 15.5; N = 30 FP64 109.0 at 5, 112.0 at 6, 110.3 at 10, 114.1 at 3, FP32 67.0 at 5 and 6, 69.3 at 3,
+// 71.8 at 10.  At N = 8, 10, 11 and 16 batches at 1, 2, 3 and 4 differ by up to 4 % either way (FP64 3-view
+// triangulation, N = 8, 3.59, 3.64, 3.64, 3.65; 4-view, N = 11, 6.63, 6.60, 6.58, 6.71; 5-point full form,
+// N = 16, 14.2, 14.4, 14.7, 14.8).
+__host__ __device__ constexpr int lu_group(int N) { return N <= 6 ? 1 : N <= 18 ? 3 : 5; }
 // stored pivot rows of a group that starts with rows of w entries: even stride (with the right-hand
 // side at entry w), so that the back substitution's diagonal reads fall into different banks
 __host__ __device__ constexpr int lu_row_stride(int w) { return (w + 2) & ~1; }
