@@ -323,6 +323,13 @@ constexpr bool kFlatAlways = N > 16;
 // only by 2 (30x30 FP64 113.3 against 118.9 ms).
 template <int N>
 constexpr int kUnrollHt = N > 16 ? 2 : 4;
+// The mixed kernel's general H_x walk at 5 unknowns only by 2: by 4 the kernel spills, and its code, with
+// the FP64 residual's general walk beside it, is longer than short lists repay (distorted 2-view
+// triangulation, 18 terms a lane, 1,428 hypotheses 8.87 -> 8.70 ms; TDOA, 45 terms, 45.3 -> 44.6); the longer
+// lists of the problems with 4 and 6 unknowns are better by 4 (PnP by quaternions 22.1 against 22.5,
+// 6-line 3-view 731 against 737).
+template <int N, int NVX, bool MIXED>
+constexpr int kUnrollHx = MIXED && NVX < 0 && N == 5 ? 2 : 4;
 
 // Row r of H (which = 0) or of -H_t (which = 1) from the H_t term table, in precision R
 template <typename R, int N, int KIND, int NVT>
@@ -351,7 +358,7 @@ __device__ __forceinline__ cx<R> eval_rhs(const uint2* terms, const uint16_t* of
   return which ? mk(-h.re, -h.im) : h;
 }
 
-template <typename R, int N, int W, int KIND, int NVX>
+template <typename R, int N, int W, int KIND, int NVX, int U>
 __device__ __forceinline__ void eval_row(const Tables& tb, const unsigned char* ca, const unsigned char* xs, int r,
                                          bool live, cx<R> (&A)[N], int walk, uint2 seg, unsigned char* scr, unsigned nz) {
   // the row's k-th non-zero entry waits in slot k (W complex values each) until the row is read back
@@ -382,7 +389,7 @@ __device__ __forceinline__ void eval_row(const Tables& tb, const unsigned char* 
     const int len = (int)(seg.x >> 16);
     const uint2* wp = tb.hx_terms + r + (seg.x & 0xffffu) * W;  // (the staged section is the balanced one)
     cx<R> acc = mk(R(0), R(0));
-#pragma unroll 4
+#pragma unroll(U)
     for (int q = 0; q < len; ++q) {
       const uint2 w = wp[q * W];
       acc = acc_term<R, NVX>(acc, term_coef_value<R, KIND, NVX>(w, ca), w, xs);
@@ -399,7 +406,7 @@ __device__ __forceinline__ void eval_row(const Tables& tb, const unsigned char* 
       const uint2* wp = tb.hx_terms + r + (seg.x & 0xffffu) * N;
       cx<R>* sp = view<R>(scr) + r + seg.y * W;
       cx<R> acc = mk(R(0), R(0));
-#pragma unroll 4
+#pragma unroll(U)
       for (int q = 0; q < len; ++q) {
         const uint2 w = wp[q * N];
         acc = acc_term<R, NVX>(acc, term_coef_value<R, KIND, NVX>(w, ca), w, xs);
@@ -870,8 +877,9 @@ __device__ __forceinline__ uint2 walk_range(const Tables& tb, int walk, int l, i
 template <typename R, typename RL, int N, int W, int KIND, int S>
 __device__ __forceinline__ void eval_any(const Tables& tb, const SubMem& sm, int l, cx<RL> (&A)[N], cx<RL>& b,
                                          int which) {
-  eval_row<RL, N, W, KIND, shape_nvx(S)>(tb, sm.coefA, sm.xs, l, l < N, A, sm.walk, reinterpret_cast<const uint2*>(sm.seg)[l],
-                                         sm.scr, sm.nz);
+  constexpr int NVX = shape_nvx(S);
+  eval_row<RL, N, W, KIND, NVX, kUnrollHx<N, NVX, !std::is_same<R, RL>::value>>(
+      tb, sm.coefA, sm.xs, l, l < N, A, sm.walk, reinterpret_cast<const uint2*>(sm.seg)[l], sm.scr, sm.nz);
   if constexpr (std::is_same<R, RL>::value) {
     b = eval_rhs<RL, N, KIND, shape_nvt(S)>(tb.ht_terms, tb.ht_off, sm.coefA, sm.coefB, sm.xs, l, l < N, which);
   } else {
