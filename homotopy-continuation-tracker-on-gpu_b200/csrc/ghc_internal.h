@@ -10,6 +10,7 @@
 // entry (row, col) for H_x and by row for H / H_t, with CSR offsets; the words
 // are stored row-interleaved (term k of row r at k * N + r).
 #pragma once
+#include <cstddef>
 #include <cstdint>
 
 #ifdef __CUDACC__
@@ -142,6 +143,26 @@ inline int eval_shape_of(int kind, int Px, int Pt) {
 }
 GHC_HD constexpr int shape_nvx(int S) { return S == EVAL_1_2 ? 1 : S == EVAL_2_3 ? 2 : -1; }
 GHC_HD constexpr int shape_nvt(int S) { return S == EVAL_1_2 ? 2 : S == EVAL_2_3 ? 3 : -1; }
+
+// CTA size (threads, a multiple of 32 up to max_block) with the most threads on an SM by shared memory and
+// by the registers that the kernel is compiled for (max_threads); `block` itself where no other has more
+// than its `threads`, and the smallest of equal ones.
+inline int widest_block(size_t tables, size_t per_sub, int W, int max_block, int max_threads, int block,
+                        int threads) {
+  constexpr size_t kPerSm = 228 * 1024, kReserved = 1024;  // shared memory of an SM, and what each CTA costs beside its own
+  int best = block, most = threads;
+  for (int b = 64; b <= max_block; b += 32) {
+    const size_t cta = tables + (size_t)(b / W) * per_sub;
+    if (cta + kReserved > kPerSm) break;  // (as much as one CTA may have: 227 KB)
+    int n = (int)(kPerSm / (cta + kReserved)) * b;
+    if (n > max_threads) n = max_threads;
+    if (n > most) {
+      most = n;
+      best = b;
+    }
+  }
+  return best;
+}
 
 // Everything the tracker kernel needs, by value.
 struct TrackParams {

@@ -29,25 +29,6 @@ inline int block_threads(size_t tables, size_t per_sub, int W) {
   return 0;
 }
 
-// CTA size (threads, a multiple of 32 up to max_block) with the most threads on an SM by shared memory;
-// `block` itself where no other has more than its `threads`, and the smallest of equal ones.  The
-// register limit is the caller's to check.
-inline int widest_block(size_t tables, size_t per_sub, int W, int max_block, int block, int threads) {
-  constexpr size_t kPerSm = 228 * 1024, kReserved = 1024;  // shared memory of an SM, and what each CTA costs beside its own
-  int best = block, most = threads;
-  for (int b = 64; b <= max_block; b += 32) {
-    const size_t cta = tables + (size_t)(b / W) * per_sub;
-    if (cta + kReserved > kPerSm) break;  // (as much as one CTA may have: 227 KB)
-    int n = (int)(kPerSm / (cta + kReserved)) * b;
-    if (n > 512) n = 512;
-    if (n > most) {
-      most = n;
-      best = b;
-    }
-  }
-  return best;
-}
-
 // A launch whose term words and path buffers do not fit into one CTA even at 32 threads reads the words
 // where they are (EVAL_IN_PLACE; the same sums in the same order).  The words then come through L1, which
 // is slower, so no other launch does; and the walk is the one that needs the least shared memory:
@@ -96,13 +77,16 @@ int launch_track_w(const TrackParams& p, cudaStream_t s, int n_sm) {
   }
   int occ = occupancy(block, 0);
   if (occ < 0) return occ;
-  if (dev::track_block<N, R, RL, V>() > kBlock && p.n_items > (long long)occ * n_sm * (block / W)) {
+  constexpr int kMaxBlock = dev::track_block<N, R, RL, V>();
+  if (kMaxBlock > kBlock && p.n_items > (long long)occ * n_sm * (block / W)) {
     // more paths than one wave of the usual CTAs: the CTA size that keeps the most paths on an SM
-    const int wide = widest_block(tables, per_sub, W, dev::track_block<N, R, RL, V>(), block, occ * block);
+    const int wide = widest_block(tables, per_sub, W, kMaxBlock, dev::track_ctas<N, R, RL, V>() * kMaxBlock, block,
+                                  occ * block);
     if (wide != block) {
       const int o = occupancy(wide, 1);
-      if (o < 0) return o;
-      if (o * wide > occ * block) {
+      if (o < 0) {
+        cudaGetLastError();  // refused: the usual CTAs then
+      } else if (o * wide > occ * block) {
         block = wide;
         occ = o;
       }
