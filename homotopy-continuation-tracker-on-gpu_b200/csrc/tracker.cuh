@@ -464,7 +464,7 @@ __device__ __forceinline__ void static_for(F&& f) {
 //               and eliminates it in its registers, rows swapped by selects: no pivot search across
 //               lanes and no broadcast per column, so a lone small system's solve is a short chain
 //               (the single-instance P3P case is latency bound).
-constexpr int LU_GROUPED = 0, LU_SERIAL = 2;
+constexpr int LU_GROUPED = 0, LU_SERIAL = 1;
 #ifndef GHC_LU_SERIAL_MAX_N
 #define GHC_LU_SERIAL_MAX_N 3
 #endif
@@ -1484,7 +1484,6 @@ __global__ void __launch_bounds__(128) polish_kernel(const PolishParams p) {
   write_one<double, double, N>(sm, l);
   reinterpret_cast<uint2*>(sm.seg)[l] = walk_range<N, W, shape_nvx(S)>(tb, walk, l, 0, 1);
   const int subs_per_cta = blockDim.x / W;
-  const int leader = lane - l;
   for (long long item0 = (long long)blockIdx.x * subs_per_cta; item0 < p.n_items;
        item0 += (long long)gridDim.x * subs_per_cta) {
     const long long item = item0 + g;
@@ -1518,13 +1517,12 @@ __global__ void __launch_bounds__(128) polish_kernel(const PolishParams p) {
     cx<double> h;
     eval_any<double, double, N, W, KIND, S>(tb, sm, l, A, h, 0);
     const double s = tree_sum<double, N, W>(l < N ? c_abs2(h) : 0.0);
-    const double s0 = __shfl_sync(kFull, s, leader);
     if (valid) {
       if (conv && l < N) {
         ep[2 * l] = x.re;
         ep[2 * l + 1] = x.im;
       }
-      if (l == 0 && p.resid) p.resid[item] = conv ? sqrt(s0) : -1.0;
+      if (l == 0 && p.resid) p.resid[item] = conv ? sqrt(s) : -1.0;
     }
     __syncwarp(kFull);
   }
