@@ -54,10 +54,9 @@ constexpr int kMaxVarsBalanced = 5;
 // lanes per path (the sub-warp width) for N unknowns
 GHC_HD constexpr int subwarp_width(int N) { return N <= 4 ? 4 : N <= 8 ? 8 : N <= 16 ? 16 : 32; }
 
-// Sizes that get the balanced H_x walk (tables and kernel code): every size.  B200, tuned: 5-point
-// (N = 6) +11 %, 30x30 (N = 30) +4 %.  (When the walk was chosen at run time inside one kernel, the
-// balanced code cost the N = 12 problems 4-5 % on their row-wise walk; each walk is its own kernel
-// now, so building it costs the other walks nothing.)
+// Sizes that get the balanced H_x walk (tables and kernel code): every size, for each walk is its own
+// kernel and costs the others nothing; where it is the default, and the times, stand at
+// flat_eval_pays().
 GHC_HD constexpr bool balanced_walk_built(int) { return true; }
 
 // The compiled H_x offsets: [N*N+1] CSR offsets of the terms per (row, column), then the

@@ -250,7 +250,9 @@ __device__ __forceinline__ void coef_loop_p2c(const double* __restrict__ hx, con
 // The lanes of a path read its tables entry by entry at a stride of K (+ 1) complex values, so every
 // load touches most lines of the table: half as many loads (whole complex values) are half as many
 // passes over them.  With the shorter path record: P3P one instance FP64 123 -> 105 us, 20,000 hypotheses
-// 2.11 -> 1.88 ms, 5-point 12.3 -> 10.9, gen-3v-4pt 90.5 -> 84.8.
+// 2.11 -> 1.88 ms, 5-point 12.3 -> 10.9, gen-3v-4pt 90.5 -> 84.8.  Higher degrees keep 8-byte loads: 16-byte
+// ones there gained 1.5 to 3.5 % on 6-point rolling shutter and P4P (K = 3), nothing on distorted 2-view
+// triangulation and TDOA, and cost 6-line 3-view 2.4 % in mixed precision.
 template <typename R, typename RO, bool HI>
 __device__ __forceinline__ void coef_eval_p2c(const double* __restrict__ hx, const double* __restrict__ ht, int M,
                                               int K, R t, bool fresh, cx<RO>* c, cx<RO>* cp, cx<R>* hi, int l, int step) {
@@ -451,15 +453,15 @@ __device__ __forceinline__ void static_for(F&& f) {
 // operations of every entry in the oracle's order:
 //   LU_GROUPED  columns in groups of lu_group(N), each group one rolled loop whose body eliminates
 //               the row's first entry and shifts the row down by one, so that a column needs no
-//               compile-time index: the code is one body per group instead of one per column
-//               (N = 12: 0.5 K instead of 1.9 K instructions).  The pivot rows stay in shared
-//               memory, where the back substitution finds them; pivoted lanes go on computing
-//               values that nothing reads, so the update has no branch.  What bounded the LU with
-//               every column unrolled was fetching its code (gen-3v-4pt: 2.0 of 8.9 cycles per
-//               issue); grouped, the same tracker issues in 62 instead of 51 % of the cycles.
-//               Measured against it (B200, default launch choice): gen-3v-4pt FP64 101.9 -> 92.8 ms
-//               (512 hypotheses), mixed 46.6 -> 39.0 (251), CY 103.2 -> 96.8 (128), 30x30 FP64
-//               126.8 -> 117.0 (48), mixed 86.8 -> 75.8 (37); 5-point equal (-0.4 %).
+//               compile-time index: the code is one body per group instead of one per column.
+//               The pivot rows stay in shared memory, where the back substitution finds them;
+//               pivoted lanes go on computing values that nothing reads, so the update has no
+//               branch.  What bounded the LU with every column unrolled was fetching its code
+//               (gen-3v-4pt: 2.0 of 8.9 cycles per issue; grouped 0.2).  Measured when it took the
+//               unrolled form's place (B200, default launch choice, groups of 2, 4 and 10 at N = 6,
+//               12 and 30): gen-3v-4pt FP64 101.9 -> 92.8 ms (512 hypotheses), mixed 46.6 -> 39.0 (251),
+//               CY 103.2 -> 96.8 (128), 30x30 FP64 126.8 -> 117.0 (48), mixed 86.8 -> 75.8 (37);
+//               5-point equal (-0.4 %).
 //   LU_SERIAL   (N <= 3) every lane of the sub-warp gathers the whole system through shared memory
 //               and eliminates it in its registers, rows swapped by selects: no pivot search across
 //               lanes and no broadcast per column, so a lone small system's solve is a short chain
@@ -639,8 +641,9 @@ __device__ __forceinline__ cx<R> lu_solve_grouped(cx<R> (&A)[N], cx<R> b, int l,
       const bool cand = pos >= i;
       // The group's later columns have shorter rows; leaving their last entries out (uniformly) spares
       // shared-memory traffic, which bounds FP64 up to 16 unknowns (gen-3v-4pt 91.9 -> 89.8 ms, CY
-      // 93.9 -> 91.9); in FP32 and at N = 30 the added branches cost more (mixed 39.5 -> 40.9,
-      // 30x30 112.9 -> 118.2).
+      // 93.9 -> 91.9; batches at N = 8, 10 and 11 equal, 5-point full form, N = 16, 14.5 -> 14.7, and one
+      // instance there 4 to 7 % slower); in FP32 and at N = 30 the added branches cost more (mixed
+      // 39.5 -> 40.9, 30x30 112.9 -> 118.2).
       constexpr bool kTrim = sizeof(R) == 8 && N > 6 && N <= 16;
       const int t = i - c0;
       auto has = [&](auto jc) {
@@ -1155,8 +1158,7 @@ __device__ __forceinline__ void track_body(const TrackParams& p, unsigned char* 
   write_one<R, RL, N>(sm, l);
   // Spread, all sub-warps of the warp have the same path: they share one copy of the coefficients and
   // of the row scratch, and each evaluates a part of both, which shortens the chain of a lone path
-  // (B200, one instance: P3P FP64 107 -> 92 us, 5-point FP32 2.19 -> 1.57 ms, gen-3v-4pt FP32
-  // 1.09 -> 1.00).  What a sub-warp updates in place, and its solve, stay its own.
+  // (B200, one instance: P3P FP64 107 -> 92 us, 5-point FP32 2.19 -> 1.57 ms).  What a sub-warp updates in place, and its solve, stay its own.
   reinterpret_cast<uint2*>(sm.seg)[l] =
       walk_range<N, W, shape_nvx(S)>(tb, walk, l, p.spread ? lane / W : 0, p.spread ? 32 / W : 1);
   if (p.spread) {
