@@ -30,9 +30,10 @@ inline int block_threads(size_t tables, size_t per_sub, int W) {
 }
 
 // A launch whose term words and path buffers do not fit into one CTA even at 32 threads reads the words
-// where they are (EVAL_IN_PLACE; the same sums in the same order).  The words then come through L1, which
-// is slower, so no other launch does; and the walk is the one that needs the least shared memory:
-// entry-wise, where that is built.
+// where they are (EVAL_IN_PLACE; the same sums in the same order).  Only such a launch: forced on others, ms,
+// entry-wise staged / in place, FP64 gen-3v-4pt 12.8 / 16.2 (51 hypotheses), CY 33.4 / 49.8 (44), 5-point
+// 6.4 / 15.4 (1,000); 6-line 3-view, whose own walk is the balanced one (658), 713 / 626 and FP32 333 / 364 (balanced
+// 313).  The walk is the one that needs the least shared memory: entry-wise, where that is built.
 constexpr int in_place_walk(int N) { return N > 16 ? 1 : 0; }
 
 template <typename R, typename RL, int N, int KIND, int V, int S, int WK>
